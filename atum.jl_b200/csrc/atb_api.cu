@@ -8,7 +8,7 @@
 #include "../../include/atum_b200.h"
 #include "atb_generic.cuh"
 #include "atb_reduce.cuh"
-#include "atb_tendency.cuh"
+#include "atb_fd.cuh"
 #include "atb_curved.cuh"
 
 #include <algorithm>
@@ -147,6 +147,7 @@ struct atb_op {
   std::vector<int> col_e0;    // bottom element of every vertical column
   bool cols_uniform = true;   // every instance has the same element counts
   int npre = 0, npv = 0;
+  bool fd = false;   // flux differencing by the flux-differencing kernels (atb_fd.cuh)
   // page-locked geometry staging of pools: a ring of kGeoRing areas, each
   // reused once the copies out of it have run, so a placement waits only for
   // the copies of the placement kGeoRing before it
@@ -156,6 +157,7 @@ struct atb_op {
   cudaEvent_t geo_ev[kGeoRing] = {};  // last copy out of h_geo[i]
   int geo_turn = 0;
   std::vector<double> w, D;
+  double cfd[64] = {};  // Cfd, Nq x Nq
   double* d_ginv = nullptr;
   int* d_nbr = nullptr;
   double* d_aux = nullptr;
@@ -191,9 +193,25 @@ namespace {
 // warps (the face tasks are spread over warp-aligned groups)
 int cta_threads(int E, int Np) { return ((E * Np + 31) / 32) * 32; }
 
-size_t op_smem(const atb_op* op, int E, int pf = 0) {
+// shared memory of the node-per-thread kernels' layout: which counts
+// atb_op_set_launch takes does not depend on the kernel that serves them
+size_t node_smem(const atb_op* op, int E) {
   if (op->curved) return curved_smem_bytes(op->vk, op->naux_used, op->Nq, E);
-  return tend_smem_bytes(op->ns, op->npre, op->naux_used, op->dim, op->Nq, op->Np, op->Nfp, E, op->npv, false, pf);
+  return tend_smem_bytes(op->ns, op->npre, op->naux_used, op->dim, op->Nq, op->Np, op->Nfp, E, op->npv);
+}
+
+// elements and threads of a tendency launch: the flux-differencing kernels are
+// compiled for at most fd_max_elements elements per CTA (the shape does not
+// change results)
+int op_elements(const atb_op* op) { return op->fd ? std::min(op->E, fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq)) : op->E; }
+int op_threads(const atb_op* op, int E) {
+  return op->fd ? fd_threads(op->Nq, op->dim, E) : cta_threads(E, op->Np);
+}
+
+size_t op_smem(const atb_op* op, int E) {
+  if (op->fd)
+    return fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, std::min(E, fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq)), false);
+  return node_smem(op, E);
 }
 
 void fill_args(const atb_op* op, TendArgs& A) {
@@ -201,8 +219,9 @@ void fill_args(const atb_op* op, TendArgs& A) {
   A.Nq = op->Nq;
   A.Np = op->Np;
   A.Nfp = op->Nfp;
-  A.E = op->E;
+  A.E = op_elements(op);
   A.naux = op->naux_used;
+  if (op->fd) std::memcpy(A.cfd, op->cfd, sizeof(A.cfd));
   A.ginv = op->d_ginv;
   A.nbr = op->d_nbr;
   A.aux = op->d_aux;
@@ -221,9 +240,9 @@ void fill_args(const atb_op* op, TendArgs& A) {
   A.adt = 0.0;
   A.lin_law = LawP{};
   A.lin_sflux = 0;
+  A.lin_gg1 = 0.0;
   A.lin_dirs = 0;
   A.naux_nl = op->naux_used;
-  A.pf = 0;
   A.Dmat = op->d_D;
   A.G = op->d_G;
   A.MJn = op->d_MJn;
@@ -261,8 +280,8 @@ int run_tendency(atb_op* op, int epi, const double* const* q, double* const* out
     A.out[s] = out ? out[s < op->ns ? s : 0] : nullptr;
     A.out2[s] = out2 ? out2[s < op->ns ? s : 0] : nullptr;
   }
-  const size_t smem = op->smem;  // plain kernels: no epilogue prefetch (A.pf = 0)
-  int grid = (op->K_active + op->E - 1) / op->E;
+  const size_t smem = op->smem;
+  int grid = (op->K_active + A.E - 1) / A.E;
   if (grid == 0) return ATB_OK;
   tend_launch_fn fn = op->launch;
   if (op->persist_ctas > 0) {
@@ -271,7 +290,7 @@ int run_tendency(atb_op* op, int epi, const double* const* q, double* const* out
   }
   {
     ProfScope ps(op->prof_class, st);
-    fn(A, grid, cta_threads(op->E, op->Np), smem, st);
+    fn(A, grid, op_threads(op, A.E), smem, st);
   }
   return check_launch("tendency");
 }
@@ -494,10 +513,9 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   }
   if (!fn) return fail(ATB_ERR_INVALID, "unsupported (law %d, volume flux %d) combination", d->law, d->volume_flux);
   const int sf = d->surface_flux;
-  if (sf == ATB_FLUX_RUSANOV) {
-    // the kernel with the surface flux built in, where one is compiled
-    if (tend_launch_fn fr = pick_launcher_rusanov(d->law, d->dim, vk, nq)) fn = fr;
-  }
+  // two-point volume fluxes: the flux-differencing kernel, where one is compiled
+  const tend_launch_fn fl = pick_fd(d->law, d->dim, vk, nq, sf);
+  if (fl) fn = fl;
   bool sf_ok = sf == ATB_FLUX_CENTRAL || sf == ATB_FLUX_RUSANOV;
   if (d->law == LAW_EULER || d->law == LAW_EG) sf_ok = sf_ok || (sf >= ATB_FLUX_EC && sf <= ATB_FLUX_MATRIX);
   if (d->law == LAW_SW) sf_ok = sf_ok || sf == ATB_FLUX_EC || sf == ATB_FLUX_ROE;
@@ -599,6 +617,11 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   op->npre = npre_of(d->law, dim, vk);
   op->npv = npv_stride_of(d->law, dim, vk);
   op->E = std::max(1, 128 / Np);
+  if (fl) {
+    op->fd = true;
+    std::copy(tab.begin(), tab.begin() + Nq * Nq, op->cfd);
+    op->E = fd_default_elements(d->law, dim, vk, Nq, K);
+  }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
   if (op->smem > 227 * 1024) {
@@ -710,6 +733,7 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
       return fail(ATB_ERR_INVALID, "curved elements: M J must be positive");
     }
   op->curved = true;
+  op->fd = false;  // its kernels and their shapes are the curved ones
   op->launch = fn;
   // aux the kernels read: Phi (fluxes, wave speeds), grad Phi (weak-form
   // gravity), the reference state (linear law; pde_level_balance)
@@ -887,7 +911,7 @@ extern "C" int atb_op_autotune(atb_op* op, const double* const* q, double* scrat
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  for (int E = 1; cta_threads(E, op->Np) <= 512 && E <= 16; ++E) {
+  for (int E = 1; op->fd ? E <= fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq) : (cta_threads(E, op->Np) <= 512 && E <= 16); ++E) {
     if (op_smem(op, E) > 200 * 1024) break;
     op->E = E;
     op->smem = op_smem(op, E);
@@ -913,7 +937,7 @@ extern "C" int atb_op_set_persistent(atb_op* op, int ctas) {
   if (!op || ctas < 0) return fail(ATB_ERR_INVALID, "bad argument");
   if (ctas > 0) {
     tend_launch_fn fn = op->curved ? nullptr
-                                   : pick_launcher_persistent(op->law.kind, op->dim, op->vk, op->Nq, op->sflux, false, 0);
+                                   : pick_fd_persistent(op->law.kind, op->dim, op->vk, op->Nq, op->sflux, false, 0);
     if (!fn)
       return fail(ATB_ERR_INVALID, "no persistent kernel for this operator (brick, Rusanov surface flux, N = 3..5: "
                                    "3-D Euler-gravity EC, 2-D Euler EC, 2-D shallow water EC / FP32-flux EC)");
@@ -925,7 +949,7 @@ extern "C" int atb_op_set_persistent(atb_op* op, int ctas) {
 
 extern "C" int atb_op_set_launch(atb_op* op, int elements_per_cta) {
   if (!op || elements_per_cta < 1 || cta_threads(elements_per_cta, op->Np) > 512 ||
-      op_smem(op, elements_per_cta) > 227 * 1024)
+      node_smem(op, elements_per_cta) > 227 * 1024)
     return fail(ATB_ERR_INVALID, "bad elements per CTA");
   op->E = elements_per_cta;
   op->smem = op_smem(op, elements_per_cta);
@@ -1434,7 +1458,7 @@ int rlsrk_step(atb_solver* s, double* const* q, cudaStream_t st) {
 // right-hand side, and no separate combination kernel runs.  The additions
 // happen in the same order as in ark_step, so the results are identical.
 // one fused ARK stage launch: explicit tendency and linear operator of Q in
-// one pass, EPI_ARK accumulation (atb_tendency.cuh, FUSE = true)
+// one pass, EPI_ARK accumulation (atb_fd.cuh, FUSE = true; curved: atb_curved.cu)
 int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t st) {
   atb_op* op = s->rhs;
   TendArgs A;
@@ -1448,8 +1472,7 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
     const size_t bytes = curved_smem_bytes(op->vk, naux, op->Nq, E, true);
     if (bytes > 227 * 1024) return fail(ATB_ERR_INVALID, "element too large for the fused curved ARK stage kernel");
     A.E = E;
-    A.pf = 0;
-    A.epi = EPI_ARK;
+      A.epi = EPI_ARK;
     A.lin_law = s->lin->law;
     A.lin_sflux = s->lin->sflux;
     A.lin_dirs = s->lin->dirs;
@@ -1472,24 +1495,14 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
     }
     return check_launch("fused curved ARK stage");
   }
-  int pf = 0;
-  for (int j = 0; j < 3; ++j) pf += (ark.acc[j][0] && ark.accin[j][0]) ? 1 : 0;
-  // the compact layout of the Nq-specialised kernels (atb_tendency.cuh)
-  const bool cmp = op->Nq >= 3 && op->Nq <= 8 && fused_compact_fits(op->Nq, op->dim, op->ns, op->npre, op->npv);
-  auto bytes = [&](int e) {
-    return tend_smem_bytes(op->ns, op->npre, naux, op->dim, op->Nq, op->Np, op->Nfp, e, op->npv, true, pf, cmp);
-  };
-  // fused kernels are compiled for fused_max_threads per CTA
-  const int maxthr = fused_max_threads(op->Nq, cmp);
-  while (E > 1 && (cta_threads(E, op->Np) > maxthr || bytes(E) > 100 * 1024)) --E;
-  if (cta_threads(E, op->Np) > maxthr) return fail(ATB_ERR_INVALID, "element too large for the fused ARK stage kernel");
-  if (pf && bytes(E) > 227 * 1024) {
-    pf = 0;  // no room: the epilogue reads its accumulators directly
-  }
+  E = op_elements(op);
+  auto bytes = [&](int e) { return fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, e, true); };
+  const size_t share = 227 * 1024 / fd_cfg(op->law.kind, op->dim, op->vk, op->Nq).min_blocks - 1024;
+  while (E > 1 && bytes(E) > share) --E;
   A.E = E;
-  A.pf = pf;
   A.epi = EPI_ARK;
   A.lin_law = s->lin->law;
+  A.lin_gg1 = A.lin_law.gamma / (A.lin_law.gamma - 1.0);
   A.lin_sflux = s->lin->sflux;
   A.lin_dirs = s->lin->dirs;
   for (int j = 0; j < 3; ++j) {
@@ -1508,7 +1521,7 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
   tend_launch_fn fn = s->fused;
   if (op->persist_ctas > 0) {
     // the persistent fused stage kernel, where one is compiled
-    if (tend_launch_fn fp = pick_launcher_persistent(op->law.kind, op->dim, op->vk, op->Nq, op->sflux, true,
+    if (tend_launch_fn fp = pick_fd_persistent(op->law.kind, op->dim, op->vk, op->Nq, op->sflux, true,
                                                      s->lin->sflux)) {
       fn = fp;
       if (grid > op->persist_ctas) grid = op->persist_ctas;
@@ -1516,7 +1529,7 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
   }
   {
     ProfScope ps(ATB_PROF_TEND, st);
-    fn(A, grid, cta_threads(E, op->Np), bytes(E), st);
+    fn(A, grid, op_threads(op, E), bytes(E), st);
   }
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess)
@@ -1874,7 +1887,7 @@ int fusion_check(atb_solver* s, cudaStream_t st) {
   const int na = R->dim + 3;
   if (R->naux < na || L->naux < na) return ATB_OK;
   tend_launch_fn f = R->curved ? pick_launcher_curved_fused(R->vk, R->sflux, L->sflux)
-                               : pick_launcher_fused(R->dim, R->vk, R->Nq, R->sflux, L->sflux);
+                               : pick_fd_fused(R->dim, R->vk, R->Nq, R->sflux, L->sflux);
   if (!f) return ATB_OK;
   unsigned long long* d_cnt = nullptr;
   int rc;
@@ -2023,7 +2036,8 @@ int atb_detail_lsrk54_steps(atb_op* op, double* const* q, double* dqbuf, double*
   bool in_user = true;
   // the same launches as the allocating path (run_tendency): the active
   // element prefix only, nothing at all when it is empty
-  const int grid = (op->K_active + op->E - 1) / op->E;
+  const int E = op_elements(op);
+  const int grid = (op->K_active + E - 1) / E;
   if (grid == 0) return ATB_OK;
   for (int step = 0; step < nsteps; ++step)
     for (int i = 0; i < 5; ++i) {
@@ -2035,7 +2049,7 @@ int atb_detail_lsrk54_steps(atb_op* op, double* const* q, double* dqbuf, double*
       for (int k = 0; k < 5; ++k) { A.q[k] = cur[k]; A.out[k] = dq[k]; A.out2[k] = oth[k]; }
       {
         ProfScope ps(op->prof_class, st);
-        op->launch(A, grid, cta_threads(op->E, op->Np), op->smem, st);
+        op->launch(A, grid, op_threads(op, E), op->smem, st);
       }
       const int rc = check_launch("tendency (no-alloc LSRK54)");
       if (rc) return rc;

@@ -83,15 +83,82 @@ template <class T> __device__ __forceinline__ T logavg_fast(T a, T b) {
   return d / dlog(a / b);
 }
 
+// 1/x for normal x: the hardware's approximation (relative error e0 <= 2^-20)
+// and one third-order step y (1 + e + e^2), e = 1 - x y (Chebyshev's iteration
+// for the reciprocal): error e0^3 = 2^-60 before the final rounding.
+__device__ __forceinline__ double rcp_cheb(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// F(u) = atanh(sqrt u) / sqrt u of the logarithmic mean (a + b) / (2 F(u)),
+// u = ((a - b) / (a + b))^2, and 1 / (2 F): polynomials interpolating them at
+// the Chebyshev nodes.  On u <= 0.00826 (a / b below 1.2) degree 5 leaves a
+// relative error under 3e-17 (the power series needs degree 7 for that); on
+// u <= 0.25 (a / b below 3) degree 13 leaves 1.7e-17.
+__device__ __forceinline__ double mean_F(double u) {
+  double s = 0.09284348541135409;
+  s = fma(u, s, 0.11109303553046275);
+  s = fma(u, s, 0.14285722052600236);
+  s = fma(u, s, 0.1999999998492953);
+  s = fma(u, s, 0.33333333333344023);
+  s = fma(u, s, 1.0);
+  return s;
+}
+__device__ __forceinline__ double mean_Gh(double u) {
+  double s = -0.011109276102071412;
+  s = fma(u, s, -0.015095031906127277);
+  s = fma(u, s, -0.02328043174345584);
+  s = fma(u, s, -0.04444444442802446);
+  s = fma(u, s, -0.16666666666667831);
+  s = fma(u, s, 0.5);
+  return s;
+}
+__device__ __forceinline__ double mean_F_wide(double u) {
+  double s = 0.2250726960064757;
+  s = fma(u, s, -0.15343412543688217);
+  s = fma(u, s, 0.1453669320455521);
+  s = fma(u, s, 0.014354447706309205);
+  s = fma(u, s, 0.05988980680927488);
+  s = fma(u, s, 0.05772990050429745);
+  s = fma(u, s, 0.06678153881929627);
+  s = fma(u, s, 0.07691472990851458);
+  s = fma(u, s, 0.09090950035823651);
+  s = fma(u, s, 0.11111109815436707);
+  s = fma(u, s, 0.14285714310189643);
+  s = fma(u, s, 0.19999999999759452);
+  s = fma(u, s, 0.33333333333334264);
+  s = fma(u, s, 1.0);
+  return s;
+}
+
+// The logarithmic mean off the short polynomial's range: the long one within a
+// factor 3, (a - b) / log(a / b) beyond.  A call: it sits in unrolled pair
+// loops that seldom reach it.
+static __device__ __noinline__ double logavg_wide(double a, double b) {
+  const double s = a + b, f = (a - b) * rcp_cheb(s), u = f * f;
+  if (u <= 0.25) return 0.5 * s * rcp_cheb(mean_F_wide(u));
+  return (a - b) / log(a / b);
+}
+
 template <class T> __device__ __forceinline__ T roe_avg(T srm, T srp, T sm, T sp) {
   return (srm * sm + srp * sp) / (srm + srp);
 }
 
 // ------------------------------------------------------------ point state
+// (FP64: the fused operations written out, so that the sum rounds the same
+// in every kernel it is inlined into)
 template <int DIM, class T> __device__ __forceinline__ T dot(const T* a, const T* b) {
   T s = a[0] * b[0];
 #pragma unroll
-  for (int d = 1; d < DIM; ++d) s = s + a[d] * b[d];
+  for (int d = 1; d < DIM; ++d) {
+    if constexpr (sizeof(T) == 8)
+      s = fma(a[d], b[d], s);
+    else
+      s = s + a[d] * b[d];
+  }
   return s;
 }
 
@@ -370,11 +437,11 @@ __device__ __forceinline__ T flux_ws_recip(const LawP& L, int d, const T* q, con
 #pragma unroll
   for (int c = 0; c < DIM; ++c) u[c] = q[1 + c] * rinv;
   if constexpr (LAW == LAW_SW) {
-    const T p = T(L.grav) * (q[0] * q[0]) / T(2);
+    const T hp = T(L.grav) * q[0] / T(2);
     f[0] = q[1 + d];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) f[1 + c] = q[1 + d] * u[c];
-    f[1 + d] = f[1 + d] + p;
+    f[1 + d] = fma(hp, q[0], f[1 + d]);
     f[DIM + 1] = u[d] * q[DIM + 1];
     return fabs(u[d]) + dsqrt(T(L.grav) * q[0]);
   } else {
@@ -386,7 +453,7 @@ __device__ __forceinline__ T flux_ws_recip(const LawP& L, int d, const T* q, con
     f[0] = q[1 + d];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) f[1 + c] = q[1 + d] * u[c];
-    f[1 + d] = f[1 + d] + dp;
+    f[1 + d] = fma(q[1 + d], u[d], dp);
     f[DIM + 1] = u[d] * (q[DIM + 1] + p);
     return fabs(u[d]) + dsqrt(g * p * rinv);
   }
@@ -449,7 +516,9 @@ template <class T> __device__ __forceinline__ T series_G(T u) {
 // series correction, so the hydrostatic balance between the pressure and
 // gravity terms is carried in FP64 while every division, logarithm and
 // advective product is FP32.  Returns FP64 row values and b_avg * rho_log.
-template <int LAW, int DIM>
+// NEAR: the caller knows that both logarithmic means of every pair it
+// evaluates are on their series branch (the same values, no branch per pair).
+template <int LAW, int DIM, bool NEAR = false>
 __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1, double b1, const float* u1,
                                          float uu1, double Phi1, double r2, double p2, double b2,
                                          const float* u2, float uu2, double Phi2, double* f, double* xtra) {
@@ -460,14 +529,14 @@ __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1
   const float ur = fr * fr, ub = fb * fb;
   double rho_log;
   float cterm;
-  if (ur < 1e-2f && ub < 1e-2f) {
+  if (NEAR || (ur < 1e-2f && ub < 1e-2f)) {
     // 1 - G(u) = u/3 + 4u^2/45 + 44u^3/945 + ... (the terms of series_G)
     const float cr = ur * (1.f / 3.f + ur * (4.f / 45.f + ur * (44.f / 945.f + ur * (428.f / 14175.f +
                      ur * (10196.f / 467775.f + ur * (10719068.f / 638512875.f + ur * (25865068.f / 1915538625.f)))))));
     rho_log = rho_avg - rho_avg * (double)cr;
     cterm = series_F(ub) * igm1 / bs;  // 1 / (2 (gamma-1) b_log)
   } else {
-    rho_log = logavg_fast(r1, r2);
+    rho_log = logavg_wide(r1, r2);
     const float b_log = (ub < 1e-2f) ? 0.5f * bs * series_G(ub) : bd / logf((float)b1 / (float)b2);
     cterm = 0.5f * igm1 / b_log;
   }
@@ -477,7 +546,11 @@ __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1
 #pragma unroll
   for (int c = 0; c < DIM; ++c) ua[c] = 0.5f * (u1[c] + u2[c]);
   const float rl = (float)rho_log;
-  const float ud = ua[d];
+  // selected, not indexed: d may be a run-time value
+  float ud = ua[0];
+#pragma unroll
+  for (int c = 1; c < DIM; ++c)
+    if (c == d) ud = ua[c];
   const float frd = ud * rl;
   f[0] = (double)frd;
   float mu = 0.f;
@@ -487,7 +560,9 @@ __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1
     f[1 + c] = (double)m;
     mu += m * ua[c];
   }
-  f[1 + d] += pc;
+#pragma unroll
+  for (int c = 0; c < DIM; ++c)
+    if (c == d) f[1 + c] += pc;
   mu += (float)pc * ud;
   float c1 = cterm - 0.25f * (uu1 + uu2);
   if (LAW == LAW_EG) c1 += (float)((Phi1 + Phi2) * 0.5);
@@ -788,9 +863,9 @@ __device__ __forceinline__ void surface_flux(const LawP& L, int kind, int d, T s
 #pragma unroll
       for (int s = 0; s < NS; ++s) nf[s] = ((fm[s] + fp[s]) / T(2)) * sgn;
       if (kind == F_RUSANOV) {
-        const T ws = dmax(wm, wp);
+        const T ws = dmax(wm, wp) / T(2);
 #pragma unroll
-        for (int s = 0; s < NS; ++s) nf[s] = nf[s] - ws * (qp[s] - qm[s]) / T(2);
+        for (int s = 0; s < NS; ++s) nf[s] = fma(-ws, qp[s] - qm[s], nf[s]);
       }
       if constexpr (LAW == LAW_SW) {
         if (L.swtopo) {  // non-conservative surface term g h- (b+ - b-)/2 n

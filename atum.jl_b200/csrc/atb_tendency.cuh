@@ -45,10 +45,6 @@
 
 namespace atb {
 
-__device__ __forceinline__ void tend_cp_async8(void* smem, const void* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
 
 // VK_EC32: the entropy-conservative volume flux in the FP32-flux precision
 // form (mixed: balance-critical terms in FP64 adds/multiplies, the rest FP32)
@@ -68,6 +64,7 @@ struct TendArgs {
   const int* nbr;      // K*6: neighbour element - e, or NBR_BOUNDARY + tag
   const double* aux;   // naux * stride
   const double* tab;   // Cfd[Nq*Nq], Cw[Nq*Nq], lift_end
+  double cfd[64];      // Cfd again for the flux-differencing kernels (Nq <= 8): constant-bank operands
   LawP law;
   int dirs, sflux, epi;
   double a, bdt;
@@ -76,12 +73,12 @@ struct TendArgs {
   double* acc[3][5];
   const double* accin[3][5];
   double ca[3], cb[3], adt;
-  // fused linear operator (tendency_kernel<..., FUSE = true>): the linear
-  // Euler-gravity law, its surface flux and directions
+  // fused linear operator (atb_fd.cuh): the linear Euler-gravity law, its
+  // surface flux and directions
   LawP lin_law;
   int lin_sflux, lin_dirs;
-  int naux_nl;  // aux components the explicit operator's faces read (fused launches stage more)
-  int pf;       // epilogue input fields prefetched into shared memory (0: read at the end)
+  double lin_gg1;  // gamma / (gamma - 1) of the linear law
+  int naux_nl;  // aux components the explicit operator's faces read
   size_t stride;      // K*Np
   // curved elements (atb_curved.cu): D[i][m], metric terms G[(d*3 + c)*stride
   // + gid] = d xi_d / d x_c, M J per node, per face node (e*6 + face)*Nfp + j
@@ -127,36 +124,14 @@ template <int LAW, int DIM, int VK> struct NPairVals {
   static constexpr int stride = v | 1;
 };
 
-// cmp: the compact layout of the fused Euler-gravity stage (fused_compact_fits)
-inline size_t tend_smem_bytes(int ns, int npre, int naux, int dim, int Nq, int Np, int Nfp, int E, int npvs,
-                              bool fuse = false, int pf = 0, bool cmp = false) {
+inline size_t tend_smem_bytes(int ns, int npre, int naux, int dim, int Nq, int Np, int Nfp, int E, int npvs) {
   const int npl = Nq * (Nq - 1) / 2;
-  size_t per;
-  if (cmp) {
-    per = (size_t)(ns + 3 + npre) * Np + (size_t)Nfp * npl * npvs + (size_t)ns * Np;
-  } else {
-    per = (size_t)(ns + naux + npre) * Np + (size_t)2 * dim * Nfp * ns;
-    if (npvs > 0) per += (size_t)Nfp * npl * npvs;
-    if (fuse) per += (size_t)ns * Np + (size_t)2 * Nfp * ns;  // linear flux rows, linear face slots
-  }
-  per += (size_t)pf * ns * Np;  // prefetched epilogue inputs
+  size_t per = (size_t)(ns + naux + npre) * Np + (size_t)2 * dim * Nfp * ns;
+  if (npvs > 0) per += (size_t)Nfp * npl * npvs;
   return sizeof(double) * (2 * (size_t)Nq * Nq + 2 + per * E) + 64 * sizeof(int);
 }
 
 __host__ __device__ constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }
-
-// Compact shared-memory layout of the fused Euler-gravity ARK stage: three
-// aux fields per node are staged (Phi, rho_ref, p_ref -- all that the volume
-// term and the face fluxes read of other nodes; grad Phi enters only the
-// linear operator's source, evaluated from registers before the face tasks),
-// the explicit face slots reuse the per-node precomputed values' region, and
-// the parked accumulators, the parked linear source and the linear face slots
-// reuse the pair buffer once the volume term is done.  It applies when those
-// regions are large enough (Nq >= 5 for the FP64 EC flux).
-__host__ __device__ constexpr bool fused_compact_fits(int nq, int dim, int ns, int npre, int npvs) {
-  return nq > 0 && npre * ipow(nq, dim) >= 2 * dim * ipow(nq, dim - 1) * ns &&
-         ipow(nq, dim - 1) * (nq * (nq - 1) / 2) * npvs >= (ns + dim) * ipow(nq, dim) + 2 * ipow(nq, dim - 1) * ns;
-}
 
 // volume-term two-point fluxes on the staged per-node layouts (row d)
 //
@@ -239,9 +214,7 @@ __device__ __forceinline__ int pair_index(int a, int b, int Nq) { return a * Nq 
 // one face-node task (face t / Nfp of direction D_, node t % Nfp): gather
 // the neighbour trace (or the boundary state), evaluate the numerical flux and
 // store it lifted into the face's shared-memory slot
-// CMPA: the staged aux fields are the compact [Phi, rho_ref, p_ref]
-// (components 0, DIM+1, DIM+2; the face fluxes read no others)
-template <int LAW, int DIM, int NAM, int D_, bool F32S = false, bool CMPA = false>
+template <int LAW, int DIM, int NAM, int D_, bool F32S = false>
 __device__ __forceinline__ void face_task(const TendArgs& A, const LawP& L, int sflux, int naux, int Nq, int Np,
                                           int Nfp, int e, int t, const double* sq, const double* sa, double* ss,
                                           double gid, double lift_end) {
@@ -256,14 +229,7 @@ __device__ __forceinline__ void face_task(const TendArgs& A, const LawP& L, int 
 #pragma unroll
   for (int s = 0; s < NS; ++s) qm[s] = sq[s * Np + nm];
 #pragma unroll
-  for (int k = 0; k < NAM; ++k) {
-    if constexpr (CMPA) {
-      const int c = (k == 0) ? 0 : (k == DIM + 1) ? 1 : (k == DIM + 2) ? 2 : -1;
-      am[k] = (k < naux && c >= 0) ? sa[c * Np + nm] : 0.0;
-    } else {
-      am[k] = (k < naux) ? sa[k * Np + nm] : 0.0;
-    }
-  }
+  for (int k = 0; k < NAM; ++k) am[k] = (k < naux) ? sa[k * Np + nm] : 0.0;
   // neighbour table entries are relative (neighbour element - e), or a
   // boundary tag offset by NBR_BOUNDARY
   const int nv = __ldg(A.nbr + 6 * e + face);
@@ -293,40 +259,11 @@ __device__ __forceinline__ void face_task(const TendArgs& A, const LawP& L, int 
 
 // NQ_ > 0: the node count per direction is a compile-time constant (index
 // arithmetic folds, line loops unroll); NQ_ = 0 reads it from the arguments.
-// CTA size limit of the fused kernels: 256 threads unless one element needs
-// more; with the compact layout at Nq = 5 (125 nodes), one element per CTA of
-// 128 threads, four CTAs per SM at the full 128-register budget (measured on
-// B200: faster than five CTAs at 96 registers, whose spills cost more than
-// the added warps gain).  cmp: the kernel uses the compact layout
-// (fused_compact_fits).
-__host__ __device__ constexpr int fused_max_threads(int nq, bool cmp = false) {
-  return (nq == 0 || nq * nq * nq > 256) ? 512 : (cmp && nq == 5) ? 128 : 256;
-}
-__host__ __device__ constexpr int fused_min_blocks(int nq, bool cmp = false) {
-  return (cmp && nq == 5) ? 4 : 512 / fused_max_threads(nq, cmp);
-}
-
-// Plain launches: up to 512 threads.  Fused launches (which carry the linear
-// operator too): fused_max_threads, with enough resident CTAs requested that
-// the register budget stays at 128 -- measured faster on B200 than the
-// spill-free 156-register allocation, whose lower occupancy costs more.
-//
-// SF >= 0: the surface flux kind (of the explicit operator and, fused, of the
-// linear one) is a compile-time constant, so the kernel carries one numerical
-// flux instead of all of them; SF = -1 reads it from the arguments.
-//
-// PERSIST: a persistent launch -- fewer CTAs than tiles of E elements, each
-// CTA walking the tiles (of every packed instance) with a grid stride and
-// restaging shared memory for each; otherwise one CTA per tile.  The tile's
-// work is the same code either way (tile_body).
-template <int LAW, int DIM, int VK, int NQ_, bool FUSE = false, int SF = -1, bool PERSIST = false>
-__global__ void __launch_bounds__(
-    FUSE ? fused_max_threads(NQ_, LAW == LAW_EG && fused_compact_fits(NQ_, DIM, NSt<LAW, DIM>::v, NPre<LAW, DIM, VK>::v,
-                                                                        NPairVals<LAW, DIM, VK>::stride))
-         : 512,
-    FUSE ? fused_min_blocks(NQ_, LAW == LAW_EG && fused_compact_fits(NQ_, DIM, NSt<LAW, DIM>::v, NPre<LAW, DIM, VK>::v,
-                                                                       NPairVals<LAW, DIM, VK>::stride))
-         : 1) tendency_kernel(const TendArgs A) {
+// The two-point fluxes of the orders and laws that are run most have kernels of
+// their own (atb_fd.cuh); this one serves the weak and central forms and every
+// other combination.
+template <int LAW, int DIM, int VK, int NQ_>
+__global__ void __launch_bounds__(512, 1) tendency_kernel(const TendArgs A) {
   constexpr int NS = NSt<LAW, DIM>::v;
   constexpr int NPRE = NPre<LAW, DIM, VK>::v;
   constexpr int NAM = NAuxMax<LAW, DIM>::v;
@@ -338,39 +275,25 @@ __global__ void __launch_bounds__(
   constexpr int NPV = PAIRS ? NPairVals<LAW, DIM, VK>::v : 0;
   constexpr int NPVS = PAIRS ? NPairVals<LAW, DIM, VK>::stride : 0;
   constexpr bool CQ = NQ_ > 0;
-  // the fused kernel runs the ARK23 stage epilogue only
-  const int epi = FUSE ? EPI_ARK : A.epi;
-  const int sflux = SF >= 0 ? SF : A.sflux;
-  const int lin_sflux = SF >= 0 ? SF : A.lin_sflux;
+  const int epi = A.epi;
+  const int sflux = A.sflux;
   extern __shared__ double sm[];
   const int Nq = CQ ? NQ_ : A.Nq;
   const int Np = CQ ? ipow(NQ_, DIM) : A.Np;
   const int Nfp = CQ ? ipow(NQ_, DIM - 1) : A.Nfp;
   const int naux = A.naux;
   const int npl = Nq * (Nq - 1) / 2;
-  constexpr bool CMP = FUSE && LAW == LAW_EG && fused_compact_fits(NQ_, DIM, NS, NPRE, NPVS);
   const int slot = threadIdx.x / Np;
   const int node = threadIdx.x - slot * Np;
   const int tabn = 2 * Nq * Nq + 2;
   double* sC = sm;            // Cfd
   double* sW = sm + Nq * Nq;  // Cw
-  const int naux_s = CMP ? 3 : naux;  // aux fields staged in shared memory
-  const size_t slotsz =
-      CMP ? (size_t)(NS + 3 + NPRE) * Np + (size_t)Nfp * npl * NPVS + (size_t)NS * Np + (size_t)A.pf * NS * Np
-          : (size_t)(NS + naux + NPRE) * Np + (size_t)2 * DIM * Nfp * NS + (size_t)Nfp * npl * NPVS +
-                (FUSE ? (size_t)NS * Np + (size_t)2 * Nfp * NS : 0) + (size_t)A.pf * NS * Np;
+  const size_t slotsz = (size_t)(NS + naux + NPRE) * Np + (size_t)2 * DIM * Nfp * NS + (size_t)Nfp * npl * NPVS;
   double* sq = sm + tabn + slot * slotsz;
   double* sa = sq + NS * Np;
-  double* sp = sa + naux_s * Np;
-  // compact: the explicit face slots take the precomputed values' region
-  double* ss = CMP ? sp : sp + NPRE * Np;
-  double* spv = CMP ? sp + NPRE * Np : ss + 2 * DIM * Nfp * NS;  // pair values
-  double* slf = spv + (size_t)Nfp * npl * NPVS;  // FUSE: linear vertical flux per node
-  // FUSE: linear z-face slots (compact: in the pair buffer, after the parked
-  // accumulators and the parked linear source)
-  double* ssl = CMP ? spv + (size_t)(NS + DIM) * Np : slf + NS * Np;
-  // prefetched epilogue inputs: the last A.pf*NS*Np doubles of the slot
-  double* spf_in = sq + slotsz - (size_t)A.pf * NS * Np;
+  double* sp = sa + naux * Np;
+  double* ss = sp + NPRE * Np;
+  double* spv = ss + 2 * DIM * Nfp * NS;  // pair values
   int* spair = (int*)(sm + tabn + A.E * slotsz);
   for (int t = threadIdx.x; t < tabn; t += blockDim.x) sm[t] = A.tab[t];
   if (PAIRS && threadIdx.x < npl) {
@@ -382,40 +305,10 @@ __global__ void __launch_bounds__(
   // everything above reads launch constants only; the state, aux and
   // accumulators below may come from the previous kernel of the stream
   pdl_wait();
-  auto tile_body = [&](const int tile) {
+  const int tile = blockIdx.x;
   const int e = tile * A.E + slot;
   const bool act = (slot < A.E) && (e < A.K);
   const size_t gid = (size_t)e * Np + node;
-  // Fused ARK stages: the epilogue's own-node inputs (the accumulators) are
-  // copied into shared memory now, asynchronously, so their latency hides
-  // behind the whole tendency; each thread later reads only what it copied.
-  // (Plain kernels keep reading them at the end: the extra code costs them
-  // registers, measured slower.)
-  if (FUSE && A.pf > 0 && act) {
-    int j = 0;
-    auto pf5 = [&](const double* p0, const double* p1, const double* p2, const double* p3, const double* p4) {
-      const double* P[5] = {p0, p1, p2, p3, p4};
-#pragma unroll
-      for (int s = 0; s < NS; ++s) tend_cp_async8(spf_in + (j * NS + s) * Np + node, P[s] + gid);
-      ++j;
-    };
-    switch (epi) {
-      case EPI_ADD: pf5(A.out[0], A.out[1], A.out[2], A.out[3], A.out[4]); break;
-      case EPI_LSRK:
-        if (A.a != 0.0) pf5(A.out[0], A.out[1], A.out[2], A.out[3], A.out[4]);
-        break;
-      case EPI_ARK:
-        if (!FUSE) pf5(A.out[0], A.out[1], A.out[2], A.out[3], A.out[4]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (A.acc[k][0] && A.accin[k][0])
-            pf5(A.accin[k][0], A.accin[k][1], A.accin[k][2], A.accin[k][3], A.accin[k][4]);
-        break;
-      case EPI_SUBOUT2:
-      case EPI_RLSRK: pf5(A.out2[0], A.out2[1], A.out2[2], A.out2[3], A.out2[4]); break;
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  }
   double qn[NS], an[NAM], Pn[NPRE > 0 ? NPRE : 1];
 #pragma unroll
   for (int k = 0; k < NAM; ++k) an[k] = 0.0;
@@ -429,13 +322,7 @@ __global__ void __launch_bounds__(
     for (int k = 0; k < NAM; ++k)
       if (k < naux) {
         an[k] = __ldg(A.aux + k * A.stride + gid);
-        if constexpr (CMP) {
-          if (k == 0) sa[node] = an[k];
-          if (k == DIM + 1) sa[Np + node] = an[k];
-          if (k == DIM + 2) sa[2 * Np + node] = an[k];
-        } else {
-          sa[k * Np + node] = an[k];
-        }
+        sa[k * Np + node] = an[k];
       }
     if constexpr (VK == VK_EC && LAW == LAW_SW) {
 #pragma unroll
@@ -512,16 +399,6 @@ __global__ void __launch_bounds__(
       }
     }
   }
-  if constexpr (FUSE && LAW == LAW_EG) {
-    // fused linear operator: its z flux rows, staged with the state (no
-    // barrier of its own)
-    if (act) {
-      double f[NS];
-      flux_dir<LAW_LEG, DIM>(A.lin_law, DIM - 1, qn, an, f);
-#pragma unroll
-      for (int s = 0; s < NS; ++s) slf[s * Np + node] = f[s];
-    }
-  }
   __syncthreads();
 
   double T[NS];
@@ -544,10 +421,6 @@ __global__ void __launch_bounds__(
     if constexpr (PAIRS) {
       // ---- phase A: each unordered pair of each line of direction d once
       if (act) {
-        // rolled: the instruction stream stays small (unrolling by two
-        // interleaves the flux chains of a thread's pairs, but the larger
-        // kernel body stalls on instruction fetch; measured 5% slower for
-        // the fused ARK stage kernel on B200)
 #pragma unroll 1
         for (int t = node; t < Nfp * npl; t += Np) {
           const int line = t / npl, p = t - line * npl;
@@ -661,34 +534,6 @@ __global__ void __launch_bounds__(
     }
   }
 
-  constexpr int DZ = DIM - 1;
-  // While the face tasks run (the register-heaviest part), the explicit
-  // accumulators wait in the pair buffer (free after the last direction) and
-  // the own-node state and aux are re-read from their staged copies
-  // afterwards: nothing of this node's stays live in registers across them.
-  constexpr bool PARK = PAIRS && CQ && ((size_t)ipow(NQ_ > 0 ? NQ_ : 1, DIM - 1) * ((NQ_ * (NQ_ - 1)) / 2) * NPVS >=
-                                        (size_t)NS * ipow(NQ_ > 0 ? NQ_ : 1, DIM));
-  if constexpr (PARK) {
-    if (act) {
-#pragma unroll
-      for (int s = 0; s < NS; ++s) spv[s * Np + node] = T[s];
-    }
-  }
-  // compact layout: the linear operator's source (it reads grad Phi, which is
-  // not staged) is evaluated now, from registers, exactly as the linear
-  // operator begins -- TL = 0, then its sources -- and parked with T; it only
-  // touches the momentum components
-  if constexpr (CMP) {
-    if (act && ((A.lin_dirs >> (DIM - 1)) & 1)) {
-      double tl[NS];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) tl[s] = 0.0;
-      add_sources<LAW_LEG, DIM>(A.lin_law, true, qn, an, tl);
-#pragma unroll
-      for (int k = 0; k < DIM; ++k) spv[(NS + k) * Np + node] = tl[1 + k];
-    }
-  }
-
   // ------------------------------------------------------------ faces
   // Face-node tasks of all elements of the CTA, spread over all its threads.
   // Where it costs little padding, each direction's 2*Nfp tasks are padded to
@@ -698,13 +543,11 @@ __global__ void __launch_bounds__(
   // flux is static.
   {
     const double lift_end = sm[2 * Nq * Nq];
-    const bool lin_faces = FUSE && LAW == LAW_EG && ((A.lin_dirs >> DZ) & 1);
-    const int naux_nl = FUSE ? A.naux_nl : naux;
     // warp-aligned groups when that costs little padding (3-D N=3, 4, 7),
     // else dense (small faces would leave most lanes idle)
     const int fpad = ((2 * Nfp + 31) / 32) * 32;
     const int fp = (10 * fpad <= 13 * 2 * Nfp) ? fpad : 2 * Nfp;
-    const int per_elem = (DIM + (lin_faces ? 1 : 0)) * fp;
+    const int per_elem = DIM * fp;
     for (int v = threadIdx.x; v < A.E * per_elem; v += blockDim.x) {
       const int es = v / per_elem, r = v - es * per_elem;
       const int dd = r / fp, tt = r - dd * fp;
@@ -712,43 +555,17 @@ __global__ void __launch_bounds__(
       if (tt >= 2 * Nfp || ef >= A.K) continue;
       double* const sqe = sm + tabn + es * slotsz;
       double* const sae = sqe + NS * Np;
-      double* const spe = sae + naux_s * Np;
-      double* const sse = CMP ? spe : spe + NPRE * Np;
-      if constexpr (FUSE && LAW == LAW_EG) {
-        if (dd == DIM) {
-          // z faces of the linear operator (face numbers 2*DZ, 2*DZ + 1): the
-          // slot pointer is shifted so those faces land in the linear slots
-          double* const ssle = CMP ? spe + NPRE * Np + (size_t)(NS + DIM) * Np
-                                   : sse + 2 * DIM * Nfp * NS + (size_t)Nfp * npl * NPVS + NS * Np;
-          face_task<LAW_LEG, DIM, NAuxMax<LAW_LEG, DIM>::v, DZ, false, CMP>(
-              A, A.lin_law, lin_sflux, naux, Nq, Np, Nfp, ef, 2 * DZ * Nfp + tt, sqe, sae,
-              ssle - (size_t)2 * DZ * Nfp * NS, __ldg(A.ginv + 3 * ef + DZ), lift_end);
-          continue;
-        }
-      }
+      double* const sse = sae + (size_t)(naux + NPRE) * Np;
       const int t = 2 * dd * Nfp + tt;
       switch (dd) {
-        case 0: face_task<LAW, DIM, NAM, 0, F32S, CMP>(A, L, sflux, naux_nl, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef), lift_end); break;
-        case 1: if constexpr (DIM > 1) face_task<LAW, DIM, NAM, 1, F32S, CMP>(A, L, sflux, naux_nl, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef + 1), lift_end); break;
-        default: if constexpr (DIM > 2) face_task<LAW, DIM, NAM, 2, F32S, CMP>(A, L, sflux, naux_nl, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef + 2), lift_end); break;
+        case 0: face_task<LAW, DIM, NAM, 0, F32S>(A, L, sflux, naux, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef), lift_end); break;
+        case 1: if constexpr (DIM > 1) face_task<LAW, DIM, NAM, 1, F32S>(A, L, sflux, naux, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef + 1), lift_end); break;
+        default: if constexpr (DIM > 2) face_task<LAW, DIM, NAM, 2, F32S>(A, L, sflux, naux, Nq, Np, Nfp, ef, t, sqe, sae, sse, __ldg(A.ginv + 3 * ef + 2), lift_end); break;
       }
     }
   }
   __syncthreads();
   if (!act) return;
-  if constexpr (PARK) {
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      T[s] = spv[s * Np + node];
-      qn[s] = sq[s * Np + node];
-    }
-    // (compact layout: nothing after this point reads the aux fields)
-    if constexpr (!CMP) {
-#pragma unroll
-      for (int k = 0; k < NAM; ++k)
-        if (k < naux) an[k] = sa[k * Np + node];
-    }
-  }
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     if (!((A.dirs >> d) & 1)) continue;
@@ -759,47 +576,7 @@ __global__ void __launch_bounds__(
 #pragma unroll
     for (int s = 0; s < NS; ++s) T[s] = T[s] - ss[(face * Nfp + j) * NS + s];
   }
-  // fused linear operator: the weak-form linear Euler-gravity operator along
-  // z, evaluated exactly as its own launch would: sources, then the D^T
-  // contraction of the staged flux rows, then the z faces
-  double TL[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) TL[s] = 0.0;
-  if constexpr (FUSE && LAW == LAW_EG) {
-    if ((A.lin_dirs >> DZ) & 1) {
-      if constexpr (CMP) {
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) TL[1 + k] = spv[(NS + k) * Np + node];
-      } else {
-        add_sources<LAW_LEG, DIM>(A.lin_law, true, qn, an, TL);
-      }
-      const int sd = (DZ == 0) ? 1 : (DZ == 1) ? Nq : Nq * Nq;
-      const int id = ijk[DZ];
-      const int base = node - id * sd;
-      const double gz = __ldg(A.ginv + 3 * e + DZ);
-#pragma unroll
-      for (int m = 0; m < (CQ ? NQ_ : 8); ++m) {
-        if (!CQ && m >= Nq) break;
-        const int nn = base + m * sd;
-        const double c = sW[id * Nq + m] * gz;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) TL[s] = TL[s] + c * slf[s * Np + nn];
-      }
-    }
-    const int id = ijk[DZ];
-    if (((A.lin_dirs >> DZ) & 1) && (id == 0 || id == Nq - 1)) {
-      const int side = (id == Nq - 1) ? 1 : 0;
-      const int j = (DZ == 0) ? ijk[1] + Nq * ijk[2] : (DZ == 1) ? ijk[0] + Nq * ijk[2] : ijk[0] + Nq * ijk[1];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) TL[s] = TL[s] - ssl[(side * Nfp + j) * NS + s];
-    }
-  }
-
   // --------------------------------------------------------- epilogue
-  const bool pfon = FUSE && A.pf > 0;
-  if (pfon) asm volatile("cp.async.wait_all;\n" ::: "memory");
-  // j-th prefetched field, state s (own node); the same order as issued
-  auto pin = [&](int j, int s) { return spf_in[(j * NS + s) * Np + node]; };
   switch (epi) {
     case EPI_SET:
 #pragma unroll
@@ -807,7 +584,7 @@ __global__ void __launch_bounds__(
       break;
     case EPI_ADD:
 #pragma unroll
-      for (int s = 0; s < NS; ++s) A.out[s][gid] = (pfon ? pin(0, s) : A.out[s][gid]) + T[s];
+      for (int s = 0; s < NS; ++s) A.out[s][gid] = A.out[s][gid] + T[s];
       break;
     case EPI_LSRK: {
       const double bdt = A.dte ? A.bdt * A.dte[e] : A.bdt;
@@ -815,7 +592,7 @@ __global__ void __launch_bounds__(
       for (int s = 0; s < NS; ++s) {
         // first stage (a = 0): the previous increment is not read, so stale
         // or never-written increment storage cannot leak into the step
-        const double dqn = (A.a != 0.0) ? A.a * (pfon ? pin(0, s) : A.out[s][gid]) + T[s] : T[s];
+        const double dqn = (A.a != 0.0) ? A.a * A.out[s][gid] + T[s] : T[s];
         A.out[s][gid] = dqn;
         A.out2[s][gid] = qn[s] + bdt * dqn;
       }
@@ -823,15 +600,14 @@ __global__ void __launch_bounds__(
     case EPI_ARK:
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
-        // fused: T = N(Q), TL = L(Q); else out holds N(Q) and T = L(Q)
-        const double E = FUSE ? T[s] - TL[s] : (pfon ? pin(0, s) : A.out[s][gid]) - T[s];
-        const double I = FUSE ? TL[s] : T[s];
-        int jj = FUSE ? 0 : 1;
+        // out holds N(Q), T = L(Q)
+        const double E = A.out[s][gid] - T[s];
+        const double I = T[s];
 #pragma unroll
         for (int j = 0; j < 3; ++j)
           if (A.acc[j][0]) {
             double base = qn[s];
-            if (A.accin[j][0]) base = pfon ? pin(jj++, s) : A.accin[j][s][gid];
+            if (A.accin[j][0]) base = A.accin[j][s][gid];
             A.acc[j][s][gid] = base + A.adt * (A.ca[j] * E + A.cb[j] * I);
           }
       }
@@ -839,7 +615,7 @@ __global__ void __launch_bounds__(
     case EPI_SUBOUT2:
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
-        const double o2 = pfon ? pin(0, s) : A.out2[s][gid];
+        const double o2 = A.out2[s][gid];
         A.out[s][gid] = T[s];
         A.out2[s][gid] = o2 - T[s];
       }
@@ -847,21 +623,11 @@ __global__ void __launch_bounds__(
     case EPI_RLSRK:
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
-        const double o2 = pfon ? pin(0, s) : A.out2[s][gid];
+        const double o2 = A.out2[s][gid];
         A.out[s][gid] = T[s];
         A.out2[s][gid] = A.a * o2 + T[s];
       }
       break;
-  }
-  };  // tile_body
-  if constexpr (PERSIST) {
-    const int ntiles = (A.K + A.E - 1) / A.E;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-      tile_body(tile);
-      __syncthreads();  // the next tile restages shared memory
-    }
-  } else {
-    tile_body(blockIdx.x);
   }
   pdl_trigger();
 }
@@ -869,36 +635,20 @@ __global__ void __launch_bounds__(
 // launcher signature used by the host dispatch table
 typedef void (*tend_launch_fn)(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st);
 
-template <int LAW, int DIM, int VK, int NQ_ = 0, bool FUSE = false, int SF = -1, bool PERSIST = false>
+template <int LAW, int DIM, int VK, int NQ_ = 0>
 void tend_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {
     // on failure the launch below reports the error
-    if (cudaFuncSetAttribute(tendency_kernel<LAW, DIM, VK, NQ_, FUSE, SF, PERSIST>,
+    if (cudaFuncSetAttribute(tendency_kernel<LAW, DIM, VK, NQ_>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
       configured = smem;
   }
-  launch_maybe_pdl(tendency_kernel<LAW, DIM, VK, NQ_, FUSE, SF, PERSIST>, dim3(grid), dim3(block), smem, st, A);
+  launch_maybe_pdl(tendency_kernel<LAW, DIM, VK, NQ_>, dim3(grid), dim3(block), smem, st, A);
 }
-
-// persistent variants (atb_op_set_persistent) of the hot configurations: the
-// explicit Rusanov kernels of 3-D Euler-gravity, 2-D Euler and 2-D shallow
-// water (FP64 and FP32 flux) and the fused Euler-gravity ARK23 stage, for
-// the orders N = 3..5; nullptr when there is none
-tend_launch_fn pick_launcher_persistent(int law, int dim, int vk, int nq, int sflux, bool fused, int lin_sflux);
-
-// Euler-gravity explicit tendency fused with the weak-form linear operator
-// along z (ARK23 stages, split_rhs = false): 3-D, EC / FP32-flux EC volume
-// flux; nullptr when there is no such kernel
-// sflux / lin_sflux: the surface fluxes of the two operators (a kernel with
-// the flux kind built in when both are Rusanov)
-tend_launch_fn pick_launcher_fused(int dim, int vk, int nq, int sflux, int lin_sflux);
 
 // generic (runtime Nq) launcher, and the compile-time-Nq specialisations
 // that exist for (law, dim, vk, nq) -- nullptr when there is none
-// the compile-time-Nq kernels with the Rusanov surface flux built in (hot
-// explicit configurations), nullptr when there is none
-tend_launch_fn pick_launcher_rusanov(int law, int dim, int vk, int nq);
 template <int LAW> tend_launch_fn pick_launcher(int dim, int vk);
 template <int LAW> tend_launch_fn pick_launcher_nq(int dim, int vk, int nq);
 
