@@ -200,18 +200,22 @@ size_t node_smem(const atb_op* op, int E) {
   return tend_smem_bytes(op->ns, op->npre, op->naux_used, op->dim, op->Nq, op->Np, op->Nfp, E, op->npv);
 }
 
-// elements and threads of a tendency launch: the flux-differencing kernels are
-// compiled for at most fd_max_elements elements per CTA (the shape does not
-// change results)
-int op_elements(const atb_op* op) { return op->fd ? std::min(op->E, fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq)) : op->E; }
+// the line-per-thread kernels (brick or curved elements): most elements per CTA
+// they are compiled for, shared memory
+int fd_limit(const atb_op* op) {
+  return op->curved ? curved_fd_elements(op->Nq) : fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq);
+}
+size_t fd_bytes(const atb_op* op, int E, bool fuse) {
+  return op->curved ? curved_fd_smem_bytes(op->Nq, E, fuse) : fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, E, fuse);
+}
+// elements and threads of a tendency launch (the shape does not change results)
+int op_elements(const atb_op* op) { return op->fd ? std::min(op->E, fd_limit(op)) : op->E; }
 int op_threads(const atb_op* op, int E) {
   return op->fd ? fd_threads(op->Nq, op->dim, E) : cta_threads(E, op->Np);
 }
 
 size_t op_smem(const atb_op* op, int E) {
-  if (op->fd)
-    return fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, std::min(E, fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq)), false);
-  return node_smem(op, E);
+  return op->fd ? fd_bytes(op, std::min(E, fd_limit(op)), false) : node_smem(op, E);
 }
 
 void fill_args(const atb_op* op, TendArgs& A) {
@@ -620,7 +624,7 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   if (fl) {
     op->fd = true;
     std::copy(tab.begin(), tab.begin() + Nq * Nq, op->cfd);
-    op->E = fd_default_elements(d->law, dim, vk, Nq, K);
+    op->E = fd_default_elements(line_count(Nq, dim), fd_limit(op), K);
   }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
@@ -701,7 +705,10 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
   atb_op* op = nullptr;
   int rc = op_create_impl(d, 1, &aux_host, &op, d->naux > 0 && !aux_host);
   if (rc) return rc;
-  tend_launch_fn fn = pick_launcher_curved(d->law, op->vk, sf);
+  // flux differencing: one thread per line (atb_curved_fd.cuh); else per node
+  tend_launch_fn fn = pick_curved_fd(d->law, op->vk, op->Nq, sf);
+  const bool fd = fn != nullptr;
+  if (!fn) fn = pick_launcher_curved(d->law, op->vk, sf);
   if (!fn) {
     atb_op_destroy(op);
     return fail(ATB_ERR_INVALID, "curved elements: no kernel for law %d, volume flux %d", d->law, d->volume_flux);
@@ -733,7 +740,8 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
       return fail(ATB_ERR_INVALID, "curved elements: M J must be positive");
     }
   op->curved = true;
-  op->fd = false;  // its kernels and their shapes are the curved ones
+  op->fd = fd;  // its kernels and their shapes are the curved ones
+  if (fd) std::memcpy(op->cfd, op->D.data(), (size_t)Nq * Nq * sizeof(double));  // D[i][m]
   op->launch = fn;
   // aux the kernels read: Phi (fluxes, wave speeds), grad Phi (weak-form
   // gravity), the reference state (linear law; pde_level_balance)
@@ -741,10 +749,10 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
   if (d->law == LAW_EG) nu = d->pde_level_balance ? 6 : (op->vk == VK_WEAK ? 4 : 1);
   if (d->law == LAW_LEG) nu = 6;
   op->naux_used = std::min(nu, op->naux);
-  op->E = std::max(1, 128 / Np);
+  op->E = fd ? fd_default_elements(line_count(Nq, 3), fd_limit(op), K) : std::max(1, 128 / Np);
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
-  if (op->smem > 227 * 1024 || cta_threads(op->E, Np) > 512) {
+  if (op->smem > 227 * 1024 || (!fd && cta_threads(op->E, Np) > 512)) {
     atb_op_destroy(op);
     return fail(ATB_ERR_INVALID, "curved elements: element too large for one CTA");
   }
@@ -911,7 +919,7 @@ extern "C" int atb_op_autotune(atb_op* op, const double* const* q, double* scrat
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  for (int E = 1; op->fd ? E <= fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq) : (cta_threads(E, op->Np) <= 512 && E <= 16); ++E) {
+  for (int E = 1; op->fd ? E <= fd_limit(op) : (cta_threads(E, op->Np) <= 512 && E <= 16); ++E) {
     if (op_smem(op, E) > 200 * 1024) break;
     op->E = E;
     op->smem = op_smem(op, E);
@@ -1458,46 +1466,17 @@ int rlsrk_step(atb_solver* s, double* const* q, cudaStream_t st) {
 // right-hand side, and no separate combination kernel runs.  The additions
 // happen in the same order as in ark_step, so the results are identical.
 // one fused ARK stage launch: explicit tendency and linear operator of Q in
-// one pass, EPI_ARK accumulation (atb_fd.cuh, FUSE = true; curved: atb_curved.cu)
+// one pass, EPI_ARK accumulation (atb_fd.cuh, FUSE = true; curved: atb_curved_fd.cuh)
 int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t st) {
   atb_op* op = s->rhs;
   TendArgs A;
   fill_args(op, A);
   const int naux = op->dim + 3;  // [Phi, grad Phi, rho_ref, p_ref] staged for both operators
   A.naux = naux;
-  int E = op->E;
-  if (op->curved) {
-    // curved elements: the explicit operator's launch shape, no prefetch
-    while (E > 1 && curved_smem_bytes(op->vk, naux, op->Nq, E, true) > 200 * 1024) --E;
-    const size_t bytes = curved_smem_bytes(op->vk, naux, op->Nq, E, true);
-    if (bytes > 227 * 1024) return fail(ATB_ERR_INVALID, "element too large for the fused curved ARK stage kernel");
-    A.E = E;
-      A.epi = EPI_ARK;
-    A.lin_law = s->lin->law;
-    A.lin_sflux = s->lin->sflux;
-    A.lin_dirs = s->lin->dirs;
-    for (int j = 0; j < 3; ++j) {
-      for (int c = 0; c < 5; ++c) { A.acc[j][c] = ark.acc[j][c]; A.accin[j][c] = ark.accin[j][c]; }
-      A.ca[j] = ark.ca[j];
-      A.cb[j] = ark.cb[j];
-    }
-    A.adt = ark.adt;
-    for (int c = 0; c < 5; ++c) {
-      A.q[c] = Q[c];
-      A.out[c] = Q[c];  // not read by the fused epilogue
-      A.out2[c] = nullptr;
-    }
-    const int grid = (op->K_active + E - 1) / E;
-    if (grid == 0) return ATB_OK;
-    {
-      ProfScope ps(ATB_PROF_TEND, st);
-      s->fused(A, grid, cta_threads(E, op->Np), bytes, st);
-    }
-    return check_launch("fused curved ARK stage");
-  }
-  E = op_elements(op);
-  auto bytes = [&](int e) { return fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, e, true); };
-  const size_t share = 227 * 1024 / fd_cfg(op->law.kind, op->dim, op->vk, op->Nq).min_blocks - 1024;
+  int E = op_elements(op);
+  auto bytes = [&](int e) { return fd_bytes(op, e, true); };
+  const size_t share =
+      op->curved ? 227 * 1024 / 2 - 1024 : 227 * 1024 / fd_cfg(op->law.kind, op->dim, op->vk, op->Nq).min_blocks - 1024;
   while (E > 1 && bytes(E) > share) --E;
   A.E = E;
   A.epi = EPI_ARK;
@@ -1886,7 +1865,7 @@ int fusion_check(atb_solver* s, cudaStream_t st) {
   if (R->curved != L->curved) return ATB_OK;
   const int na = R->dim + 3;
   if (R->naux < na || L->naux < na) return ATB_OK;
-  tend_launch_fn f = R->curved ? pick_launcher_curved_fused(R->vk, R->sflux, L->sflux)
+  tend_launch_fn f = R->curved ? pick_curved_fd_fused(R->vk, R->Nq, R->sflux, L->sflux)
                                : pick_fd_fused(R->dim, R->vk, R->Nq, R->sflux, L->sflux);
   if (!f) return ATB_OK;
   unsigned long long* d_cnt = nullptr;

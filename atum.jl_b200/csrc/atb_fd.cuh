@@ -108,8 +108,7 @@ inline int fd_max_elements(int law, int dim, int vk, int nq) {
 // Elements per CTA when nothing else asks for a count: the fullest last warp
 // among CTAs of at least 96 threads (the smallest such), but no fewer CTAs than
 // SMs where the operator has the elements for it.
-inline int fd_default_elements(int law, int dim, int vk, int nq, int K) {
-  const int nl = line_count(nq, dim), emax = fd_max_elements(law, dim, vk, nq);
+inline int fd_default_elements(int nl, int emax, int K) {
   int best = emax;
   double fill = 0.0;
   for (int E = 1; E <= emax; ++E) {
