@@ -1081,7 +1081,7 @@ struct atb_solver {
   // operator), when the two operators allow it (atb_solver_fuse)
   tend_launch_fn fused = nullptr;
   bool fuse_on = false;
-  int lines_sparse = 0;  // per-line factors couple elements through face nodes only
+  int lines_sparse = 0;  // band: the stream of nonzero entries of per-line factors (launch_line_stream)
   // per-element time steps (LSRK over packed instances), or null; owned by
   // the solver (atb_solver_set_instance_dt) or by the caller
   double* d_dte = nullptr;
@@ -1253,7 +1253,7 @@ int build_band(atb_solver* s, cudaStream_t st) {
     launch_band_factor(M.nunk, M.bw, M.nlines, s->band, W, M.nlines, scale, st);
     s->ld = M.nlines;
     // the face-node coupling structure of every line's factor lets the solve
-    // skip the zero blocks (ATB_BAND_DENSE=1 keeps the full band)
+    // leave the zero blocks out (ATB_BAND_DENSE=1 keeps the full band)
     int* d_bad = nullptr;
     if ((rc = dalloc(&d_bad, 1))) return rc;
     CK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
@@ -1263,7 +1263,23 @@ int build_band(atb_solver* s, cudaStream_t st) {
     CK(cudaStreamSynchronize(st));
     cudaFree(d_bad);
     const char* dense = std::getenv("ATB_BAND_DENSE");
-    s->lines_sparse = (bad == 0 && !(dense && dense[0] == '1')) ? 1 : 0;
+    const size_t sn = line_stream_doubles(M);
+    if (bad == 0 && sn > 0 && !(dense && dense[0] == '1')) {
+      // the nonzero entries as each warp's stream instead of the band; without
+      // the memory to hold both for a moment the solve reads the band
+      double* stream = nullptr;
+      if (cudaMalloc(&stream, sn * sizeof(double)) == cudaSuccess) {
+        if (launch_line_stream(M, s->band, stream, st) != cudaSuccess) {
+          cudaFree(stream);
+          return fail(ATB_ERR_CUDA, "laying out the band factor failed");
+        }
+        cudaFree(s->band);
+        s->band = stream;
+        s->lines_sparse = 1;
+      } else {
+        cudaGetLastError();  // the failed allocation is not the caller's error
+      }
+    }
   } else {
     cudaFree(P);
     cudaFree(LP);

@@ -15,7 +15,8 @@
 //   band_solve_mma_kernel    the same over dense blocks, one warp per 8 rows
 //   band_solve_rows_kernel   one-state laws
 //   band_solve_shared_kernel substitution over the shared factor (below)
-// and launch_band_solve_generic (atb_generic.cu) for a factor per line.
+//   band_solve_stream_kernel, band_solve_lines_kernel  a factor per line
+// and launch_band_solve_generic (atb_generic.cu) for what is left.
 //
 // band_solve_shared_kernel: one thread owns one line; its window of solution
 // values is two register arrays (previous / current element) with every index
@@ -29,6 +30,7 @@
 #include <cstdlib>
 #include <type_traits>
 #include <utility>
+#include <vector>
 
 namespace atb {
 
@@ -1019,19 +1021,35 @@ namespace {
 
 // ------------------------------------------------ per-line factors
 // Vertical lines whose factors differ (curved grids: every column of a sphere
-// has its own metric terms).  One thread per line, the factor in the
-// line-fastest layout band[(r * W + k) * nlines + line] (coalesced across the
-// threads of a warp), the element-block recurrence with compile-time block
-// size BW1 = NQ * NS so that the previous / next block's values and the
-// current block's live in registers.  Sums run in the generic kernel's order
-// (increasing column), so the results are the generic kernel's; with SPARSE
-// the entries that the face-node coupling makes zero (the sub-diagonal block
-// of L outside its face rows and columns, the super-diagonal block of U
-// likewise; launch_band_lines_structure checks every line at setup) are not
-// read, which halves the bytes of a solve.
+// has its own metric terms).  One thread per line; every factor entry is used
+// once, so the solve is bound by reading them.  The element-block recurrence
+// has compile-time block size BW1 = NQ * NS, so that the previous / next
+// block's values and the current block's live in registers; sums run in the
+// generic kernel's order (increasing column), so the results are the generic
+// kernel's.
+//
+// band_solve_stream_kernel: factors that couple neighbouring elements through
+// face nodes only (launch_band_lines_structure checks every line at setup; the
+// other entries of those blocks, half of the band, are exact zeros).  The
+// nonzero entries are laid out once, at setup, in the order in which the solve
+// uses them, 32 lines (one warp) side by side: a warp reads one contiguous
+// stream.  It copies chunks of 16 entries (4 KB) into its own ring of eight with
+// 16-byte cp.async, seven chunks ahead, the first ones before it waits for the
+// previous kernel: 28 KB in flight per warp, 130 KB per SM at 4.6 warps, with
+// no register spent on it.  Warps are independent: one per CTA, no CTA barrier.
+// Measured on B200, 600 columns of 36 lines, 5 elements at N = 5 (21600 lines,
+// 0.83 GB of factors, 0.92 GB in all): 372 us reading the band through
+// registers (2.5 TB/s), 153 us here (6.0 TB/s; the copy bandwidth allows 142);
+// chunks of 8: the same kernel time, 19 us more per step of two solves (less
+// is read before the wait); a ring of 5 such chunks 164 us.
+//
+// band_solve_lines_kernel: any band, the factor in the line-fastest layout
+// band[(r * W + k) * nlines + line]; for coupling structures other than the
+// above.
+
 // one row of the forward (FWD) or backward pass, then the next: compile-time
 // row indices keep every block value in a register
-template <int NQ, int NS, bool SPARSE, bool FWD, int I>
+template <int NQ, int NS, bool FWD, int I>
 __device__ __forceinline__ void lines_rows(const BandSolve& B, const double* __restrict__ row0, size_t ld,
                                            size_t eoff, int nh, bool has_nb, const double (&nb)[NQ * NS],
                                            double (&cur)[NQ * NS]) {
@@ -1049,35 +1067,29 @@ __device__ __forceinline__ void lines_rows(const BandSolve& B, const double* __r
         if (k < B.npairs) acc = acc + B.dt * (B.a[k] * B.ex[k][s][g] + B.b[k] * B.im[k][s][g]);
       if (has_nb) {
 #pragma unroll
-        for (int jp = I + 1; jp < BW1; ++jp) {
-          if (SPARSE && !(I < NS && jp >= BW1 - NS)) continue;
-          acc = acc - row[(size_t)(jp - I - 1) * ld] * nb[jp];
-        }
+        for (int jp = I + 1; jp < BW1; ++jp) acc = acc - row[(size_t)(jp - I - 1) * ld] * nb[jp];
       }
 #pragma unroll
       for (int jp = 0; jp < I; ++jp) acc = acc - row[(size_t)(jp - I + BW) * ld] * cur[jp];
       cur[I] = acc;
       B.out[s][g] = acc;
-      lines_rows<NQ, NS, SPARSE, FWD, I + 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
+      lines_rows<NQ, NS, FWD, I + 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
     } else {
       double acc = B.out[s][g];
 #pragma unroll
       for (int jp = I + 1; jp < BW1; ++jp) acc = acc - row[(size_t)(jp - I + BW) * ld] * cur[jp];
       if (has_nb) {
 #pragma unroll
-        for (int jp = 0; jp < I; ++jp) {
-          if (SPARSE && !(I >= BW1 - NS && jp < NS)) continue;
-          acc = acc - row[(size_t)(2 * BW1 - 1 + jp - I) * ld] * nb[jp];
-        }
+        for (int jp = 0; jp < I; ++jp) acc = acc - row[(size_t)(2 * BW1 - 1 + jp - I) * ld] * nb[jp];
       }
       cur[I] = acc / row[(size_t)BW * ld];
       B.out[s][g] = cur[I];
-      lines_rows<NQ, NS, SPARSE, FWD, I - 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
+      lines_rows<NQ, NS, FWD, I - 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
     }
   }
 }
 
-template <int NQ, int NS, bool SPARSE>
+template <int NQ, int NS>
 __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B) {
   constexpr int BW1 = NQ * NS;
   constexpr int BW = BW1 - 1;
@@ -1099,7 +1111,7 @@ __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B)
   // forward: L y = rhs (unit diagonal)
   for (int ev = 0; ev < KV; ++ev) {
     const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
-    lines_rows<NQ, NS, SPARSE, true, 0>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev > 0, nb, cur);
+    lines_rows<NQ, NS, true, 0>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev > 0, nb, cur);
 #pragma unroll
     for (int j = 0; j < BW1; ++j) nb[j] = cur[j];
   }
@@ -1108,32 +1120,210 @@ __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B)
   for (int j = 0; j < BW1; ++j) nb[j] = 0.0;
   for (int ev = KV - 1; ev >= 0; --ev) {
     const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
-    lines_rows<NQ, NS, SPARSE, false, BW1 - 1>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev < KV - 1, nb,
-                                               cur);
+    lines_rows<NQ, NS, false, BW1 - 1>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev < KV - 1, nb, cur);
 #pragma unroll
     for (int j = 0; j < BW1; ++j) nb[j] = cur[j];
   }
   pdl_trigger();
 }
 
-typedef void (*lines_fn)(const BandSolve& B, cudaStream_t st);
-template <int NQ, int NS, bool SPARSE> void lines_launch(const BandSolve& B, cudaStream_t st) {
-  launch_maybe_pdl(band_solve_lines_kernel<NQ, NS, SPARSE>, dim3((B.M.nlines + 63) / 64), dim3(64), 0, st, B);
+// The stream of one warp (32 lines), in entries of 32 doubles: per element
+// block, forward pass bottom up, then backward pass top down, each padded to
+// whole chunks.  Forward row I: its NS entries of the previous block (I < NS),
+// then columns 0 .. I-1; backward row I = BW1-1 .. 0: columns I+1 .. BW1-1, its
+// NS entries of the next block (I >= BW1-NS), the diagonal.
+constexpr int LCHUNK = 16;  // entries per chunk
+constexpr int LRING = 8;  // chunks in the ring
+template <int NQ, int NS> struct LineStream {
+  static constexpr int BW1 = NQ * NS;
+  static constexpr int NF = BW1 * (BW1 - 1) / 2 + NS * NS, NB = NF + BW1;
+  static constexpr int CF = (NF + LCHUNK - 1) / LCHUNK, CB = (NB + LCHUNK - 1) / LCHUNK;  // chunks
+};
+// entries of one block's pass in stream order: I * W + k of the band, -1 padding
+std::vector<int> stream_order(int BW1, int NS, bool fwd) {
+  const int BW = BW1 - 1, W = 2 * BW + 1;
+  std::vector<int> o;
+  for (int r = 0; r < BW1; ++r) {
+    const int I = fwd ? r : BW1 - 1 - r;
+    if (fwd) {
+      if (I < NS)
+        for (int jp = BW1 - NS; jp < BW1; ++jp) o.push_back(I * W + jp - I - 1);
+      for (int jp = 0; jp < I; ++jp) o.push_back(I * W + jp - I + BW);
+    } else {
+      for (int jp = I + 1; jp < BW1; ++jp) o.push_back(I * W + jp - I + BW);
+      if (I >= BW1 - NS)
+        for (int jp = 0; jp < NS; ++jp) o.push_back(I * W + 2 * BW1 - 1 + jp - I);
+      o.push_back(I * W + BW);
+    }
+  }
+  while (o.size() % LCHUNK) o.push_back(-1);
+  return o;
 }
-template <int NS, bool SPARSE> lines_fn pick_lines_sp(int nq) {
+
+// order: the forward pass's nf entries, then the backward pass's nb
+__global__ void line_stream_kernel(const LineMap M, const double* band, const int* order, int nf, int nb, double* out,
+                                   size_t total) {
+  const int BW1 = M.Nq * M.ns, W = 2 * BW1 - 1;
+  const size_t per = (size_t)M.KV * (nf + nb);  // entries of a warp's stream
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    const size_t wg = (t / 32) / per, r = (t / 32) - wg * per;
+    const size_t line = wg * 32 + t % 32;
+    const bool fwd = r < (size_t)M.KV * nf;
+    const size_t rb = fwd ? r : r - (size_t)M.KV * nf;
+    const int n = fwd ? nf : nb, blk = (int)(rb / n), ev = fwd ? blk : M.KV - 1 - blk;
+    const int o = order[(fwd ? 0 : nf) + (int)(rb - (size_t)blk * n)];
+    double v = 0.0;
+    if (o >= 0) v = line < (size_t)M.nlines ? band[((size_t)ev * BW1 * W + o) * M.nlines + line] : 1.0;
+    out[t] = v;
+  }
+}
+
+struct StreamRing {
+  double* ring;       // [LRING][LCHUNK][32]
+  const double* src;  // the warp's stream
+  int nch, c;         // chunks in all, next chunk
+  const double* cur;  // this lane's entries of the current chunk
+  __device__ __forceinline__ void issue(int k) {
+    if (k < nch) {
+      const double* s = src + (size_t)k * (LCHUNK * 32) + 2 * threadIdx.x;
+      double* d = ring + (k % LRING) * (LCHUNK * 32) + 2 * threadIdx.x;
+#pragma unroll
+      for (int i = 0; i < LCHUNK / 2; ++i) cp_async16(d + 64 * i, s + 64 * i);
+    }
+    cp_async_commit();
+  }
+  // chunk c has arrived; the slot of chunk c - 1, which every lane has read, is
+  // refilled
+  __device__ __forceinline__ void next() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(LRING - 2) : "memory");
+    __syncwarp();
+    cur = ring + (c % LRING) * (LCHUNK * 32) + threadIdx.x;
+    issue(c + LRING - 1);
+    ++c;
+  }
+  // entry p of a pass (p a compile-time constant in unrolled code)
+  __device__ __forceinline__ double get(int p) {
+    if (p % LCHUNK == 0) next();
+    return cur[(p % LCHUNK) * 32];
+  }
+};
+
+// rows I, I + 1, .. (FWD) or I, I - 1, .. of one block; on entry cur holds the
+// right-hand side
+template <int NQ, int NS, bool FWD, int I>
+__device__ __forceinline__ void stream_rows(StreamRing& R, const double (&nb)[NQ * NS], double (&cur)[NQ * NS]) {
+  constexpr int BW1 = NQ * NS;
+  if constexpr (I >= 0 && I < BW1) {
+    double acc = cur[I];
+    if constexpr (FWD) {
+      constexpr int p0 = I * (I - 1) / 2 + (I < NS ? I : NS) * NS;
+      if constexpr (I < NS) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j) acc = fma(-R.get(p0 + j), nb[BW1 - NS + j], acc);
+      }
+#pragma unroll
+      for (int jp = 0; jp < I; ++jp) acc = fma(-R.get(p0 + (I < NS ? NS : 0) + jp), cur[jp], acc);
+      cur[I] = acc;
+      stream_rows<NQ, NS, FWD, I + 1>(R, nb, cur);
+    } else {
+      constexpr int r = BW1 - 1 - I;  // rows done
+      constexpr int p0 = r * (r - 1) / 2 + r + (r < NS ? r : NS) * NS;
+#pragma unroll
+      for (int j = 0; j < r; ++j) acc = fma(-R.get(p0 + j), cur[I + 1 + j], acc);
+      if constexpr (r < NS) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j) acc = fma(-R.get(p0 + r + j), nb[j], acc);
+      }
+      cur[I] = acc / R.get(p0 + r + (r < NS ? NS : 0));
+      stream_rows<NQ, NS, FWD, I - 1>(R, nb, cur);
+    }
+  }
+}
+
+template <int NQ, int NS>
+__global__ void __launch_bounds__(32) band_solve_stream_kernel(const BandSolve B) {
+  using LS = LineStream<NQ, NS>;
+  constexpr int BW1 = LS::BW1;
+  __shared__ __align__(16) double ring[LRING * LCHUNK * 32];
+  const LineMap& M = B.M;
+  const int KV = M.KV, nh = M.nh, Np = M.Np;
+  const int own = blockIdx.x * 32 + threadIdx.x;
+  const bool store = own < M.nlines;
+  const int line = store ? own : M.nlines - 1;
+  StreamRing R;
+  R.ring = ring;
+  R.nch = KV * (LS::CF + LS::CB);
+  R.src = B.band + (size_t)blockIdx.x * R.nch * (LCHUNK * 32);
+  R.c = 0;
+#pragma unroll 1
+  for (int k = 0; k < LRING - 1; ++k) R.issue(k);
+  const int hn = line % nh;
+  const int e0 = M.e0[line];
+  double nb[BW1], cur[BW1];
+#pragma unroll
+  for (int j = 0; j < BW1; ++j) nb[j] = 0.0;
+  // the right-hand side may come from the previous kernel of the stream
+  // (programmatic dependent launch, launch_maybe_pdl)
+  pdl_wait();
+  // forward: L y = rhs (unit diagonal); the first block's entries of a
+  // previous block meet nb = 0
+#pragma unroll 1
+  for (int ev = 0; ev < KV; ++ev) {
+    const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
+#pragma unroll
+    for (int j = 0; j < BW1; ++j) cur[j] = B.q[j % NS][eoff + (size_t)nh * (j / NS)];
+    for (int k = 0; k < B.npairs; ++k) {
+#pragma unroll
+      for (int j = 0; j < BW1; ++j) {
+        const size_t g = eoff + (size_t)nh * (j / NS);
+        cur[j] = cur[j] + B.dt * (B.a[k] * B.ex[k][j % NS][g] + B.b[k] * B.im[k][j % NS][g]);
+      }
+    }
+    stream_rows<NQ, NS, true, 0>(R, nb, cur);
+#pragma unroll
+    for (int j = 0; j < BW1; ++j) {
+      nb[j] = cur[j];
+      if (store) B.out[j % NS][eoff + (size_t)nh * (j / NS)] = cur[j];
+    }
+  }
+  // backward: U x = y
+#pragma unroll
+  for (int j = 0; j < BW1; ++j) nb[j] = 0.0;
+#pragma unroll 1
+  for (int ev = KV - 1; ev >= 0; --ev) {
+    const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
+    if (ev < KV - 1) {  // (the top block's y is still here)
+#pragma unroll
+      for (int j = 0; j < BW1; ++j) cur[j] = store ? B.out[j % NS][eoff + (size_t)nh * (j / NS)] : 0.0;
+    }
+    stream_rows<NQ, NS, false, BW1 - 1>(R, nb, cur);
+#pragma unroll
+    for (int j = 0; j < BW1; ++j) {
+      nb[j] = cur[j];
+      if (store) B.out[j % NS][eoff + (size_t)nh * (j / NS)] = cur[j];
+    }
+  }
+  pdl_trigger();
+}
+
+typedef void (*lines_fn)(const BandSolve& B, cudaStream_t st);
+template <int NQ, int NS> void lines_launch(const BandSolve& B, cudaStream_t st) {
+  if (B.lines_sparse)
+    launch_maybe_pdl(band_solve_stream_kernel<NQ, NS>, dim3((B.M.nlines + 31) / 32), dim3(32), 0, st, B);
+  else
+    launch_maybe_pdl(band_solve_lines_kernel<NQ, NS>, dim3((B.M.nlines + 63) / 64), dim3(64), 0, st, B);
+}
+template <int NS> lines_fn pick_lines(int nq) {
   switch (nq) {
-    case 2: return lines_launch<2, NS, SPARSE>;
-    case 3: return lines_launch<3, NS, SPARSE>;
-    case 4: return lines_launch<4, NS, SPARSE>;
-    case 5: return lines_launch<5, NS, SPARSE>;
-    case 6: return lines_launch<6, NS, SPARSE>;
-    case 7: return lines_launch<7, NS, SPARSE>;
-    case 8: return lines_launch<8, NS, SPARSE>;
+    case 2: return lines_launch<2, NS>;
+    case 3: return lines_launch<3, NS>;
+    case 4: return lines_launch<4, NS>;
+    case 5: return lines_launch<5, NS>;
+    case 6: return lines_launch<6, NS>;
+    case 7: return lines_launch<7, NS>;
+    case 8: return lines_launch<8, NS>;
   }
   return nullptr;
-}
-template <int NS> lines_fn pick_lines(int nq, bool sparse) {
-  return sparse ? pick_lines_sp<NS, true>(nq) : pick_lines_sp<NS, false>(nq);
 }
 
 __global__ void band_lines_structure_kernel(const LineMap M, const double* band, int* count) {
@@ -1163,6 +1353,31 @@ void launch_band_lines_structure(const LineMap& M, const double* band, int* coun
   band_lines_structure_kernel<<<148 * 8, 256, 0, st>>>(M, band, count);
 }
 
+size_t line_stream_doubles(const LineMap& M) {
+  if ((M.ns != 4 && M.ns != 5) || M.Nq < 2 || M.Nq > 8) return 0;
+  const int BW1 = M.Nq * M.ns;
+  const size_t per = stream_order(BW1, M.ns, true).size() + stream_order(BW1, M.ns, false).size();
+  return (size_t)((M.nlines + 31) / 32) * 32 * M.KV * per;
+}
+
+cudaError_t launch_line_stream(const LineMap& M, const double* band, double* out, cudaStream_t st) {
+  const int BW1 = M.Nq * M.ns;
+  std::vector<int> o = stream_order(BW1, M.ns, true);
+  const int nf = (int)o.size();
+  const std::vector<int> ob = stream_order(BW1, M.ns, false);
+  o.insert(o.end(), ob.begin(), ob.end());
+  int* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, o.size() * sizeof(int));
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpy(d, o.data(), o.size() * sizeof(int), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    line_stream_kernel<<<148 * 8, 256, 0, st>>>(M, band, d, nf, (int)ob.size(), out, line_stream_doubles(M));
+    e = cudaStreamSynchronize(st);
+  }
+  cudaFree(d);
+  return e;
+}
+
 bool pdl_enabled() {
   static const int on = [] {
     const char* e = std::getenv("ATB_PDL");
@@ -1173,7 +1388,7 @@ bool pdl_enabled() {
 
 void launch_band_solve(const BandSolve& B, cudaStream_t st) {
   if (B.ld > 1 && B.ld == B.M.nlines && B.npairs <= 2 && (B.M.ns == 4 || B.M.ns == 5)) {
-    lines_fn f = B.M.ns == 4 ? pick_lines<4>(B.M.Nq, B.lines_sparse != 0) : pick_lines<5>(B.M.Nq, B.lines_sparse != 0);
+    lines_fn f = B.M.ns == 4 ? pick_lines<4>(B.M.Nq) : pick_lines<5>(B.M.Nq);
     if (f) {
       f(B, st);
       return;
