@@ -517,7 +517,7 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   }
   if (!fn) return fail(ATB_ERR_INVALID, "unsupported (law %d, volume flux %d) combination", d->law, d->volume_flux);
   const int sf = d->surface_flux;
-  // two-point volume fluxes: the flux-differencing kernel, where one is compiled
+  // the line-per-thread kernel, where one is compiled
   const tend_launch_fn fl = pick_fd(d->law, d->dim, vk, nq, sf);
   if (fl) fn = fl;
   bool sf_ok = sf == ATB_FLUX_CENTRAL || sf == ATB_FLUX_RUSANOV;
@@ -623,7 +623,8 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   op->E = std::max(1, 128 / Np);
   if (fl) {
     op->fd = true;
-    std::copy(tab.begin(), tab.begin() + Nq * Nq, op->cfd);
+    // Cfd, or Cw for the weak form
+    std::copy_n(tab.begin() + (vk == VK_WEAK ? Nq * Nq : 0), Nq * Nq, op->cfd);
     op->E = fd_default_elements(line_count(Nq, dim), fd_limit(op), K);
   }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;

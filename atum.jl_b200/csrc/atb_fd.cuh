@@ -2,12 +2,12 @@
 // B200 against the node-per-thread form that stored every pair in shared
 // memory: 16^3 elements at N = 4, fused ARK23 stage 88.5 -> 44 us; 32^3 at
 // N = 7, 5.11 -> 1.66 ms; 128 shallow-water basins of 32^2 at N = 4, FP32
-// flux, 267 -> 114 us per LSRK stage.)
+// flux, 267 -> 114 us per LSRK stage; weak form, 24^3 at N = 4: 206 -> 76 us.)
 //
 // The same stage as atb_tendency.cuh's kernel (volume term, surface term,
 // sources, the stepper's write-back; the fused ARK23 stage with the weak-form
-// linear operator along z), for the two-point volume fluxes at the compiled
-// orders (2 <= Nq <= 8).
+// linear operator along z), for the two-point volume fluxes and the weak form of
+// 3-D Euler-gravity, at the compiled orders (2 <= Nq <= 8).
 //
 // What bounds it: the FP64 pipe (64 lanes per SM: one warp instruction per two
 // cycles and scheduler) and, around it, the latency of the staging loads.  The
@@ -59,15 +59,17 @@ template <int LAW, int DIM, int VK> struct LineShape {
   // a third quantity per node pair, contracted like the flux and scaled by a
   // node value at the end: the gravity fluctuation (EG) or the bathymetry
   // difference (shallow water)
-  static constexpr bool XTRA = EG || SW;
+  static constexpr bool XTRA = (EG || SW) && VK != VK_WEAK;
   // point values per node, in doubles:
   //   EC (Euler, EG)  u/2 (DIM), B = rho/p, p/rho [, Phi/4]
   //   KG              u/2 (DIM), p/2, e/2 [, Phi/4]
   //   EC32            p, b = rho/2p, p/rho [, Phi], then FP32 u (DIM), |u|^2
   //   KG32            p [, Phi], then FP32 u (DIM), e
+  //   WEAK (EG)       1/rho, p (less the reference), rho e + p, Phi/4
   //   EC (SW)         u/2 (DIM), theta/2, b
   //   EC32 (SW)       b, then FP32 u (DIM), theta
-  static constexpr int ND = SW ? (F32 ? 1 : DIM + 2)
+  static constexpr int ND = VK == VK_WEAK ? 4
+                               : SW ? (F32 ? 1 : DIM + 2)
                                : (VK == VK_EC32) ? 3 + (EG ? 1 : 0) : (VK == VK_KG32) ? 1 + (EG ? 1 : 0)
                                                                                        : DIM + 2 + (EG ? 1 : 0);
   static constexpr int NF = F32 ? DIM + 1 : 0;  // FP32 values
@@ -94,6 +96,10 @@ struct FdCfg {
 __host__ __device__ constexpr FdCfg fd_cfg(int law, int dim, int vk, int nq) {
   const bool f32 = vk == VK_EC32 || vk == VK_KG32;
   if (dim == 2) return law == LAW_SW ? FdCfg{160, nq <= 5 ? 4 : 3, 1} : FdCfg{224, 2, 2};
+  // weak form: little arithmetic, so more CTAs for the memory (24^3 elements, N =
+  // 4: 75 us at 4 of 160 threads and one array, 82 at 3 and three arrays, 95 at
+  // 8 of 96, 102 at 5 of 160; N = 1: 109 us at 8 of 96, 132 at 4 of 160)
+  if (vk == VK_WEAK && nq <= 5) return nq == 2 ? FdCfg{96, 8, 1} : FdCfg{160, 4, 1};
   if (nq == 8) return FdCfg{192, 2, 1};
   if (nq == 7) return FdCfg{160, 3, 1};
   if (nq == 6) return FdCfg{128, 4, 1};
@@ -131,7 +137,7 @@ inline int fd_nx(int law, int dim, int vk) {
   const int ns = dim + 2;
   const bool f32 = vk == VK_EC32 || vk == VK_KG32;
   const int eg = law == LAW_EG ? 1 : 0;
-  const int nd = law == LAW_SW ? (f32 ? 1 : dim + 2) : vk == VK_EC32 ? 3 + eg : vk == VK_KG32 ? 1 + eg : dim + 2 + eg;
+  const int nd = vk == VK_WEAK ? 4 : law == LAW_SW ? (f32 ? 1 : dim + 2) : vk == VK_EC32 ? 3 + eg : vk == VK_KG32 ? 1 + eg : dim + 2 + eg;
   const int nx = nd + (f32 ? (dim + 2) / 2 : 0);
   return nx > ns ? nx : ns;
 }
@@ -328,6 +334,29 @@ __device__ __forceinline__ void line_pairs(const TendArgs& A, double c0, const d
         }
       }
     }
+  }
+}
+
+// Weak form: D^T-weighted flux rows of the line's nodes (Cw in the parameters),
+// [m_n, m u_n + p n, (rho e + p) u_n] rotated
+template <int DIM, int NQ>
+__device__ __forceinline__ void line_weak(const TendArgs& A, const double* sq, const double* sx, int base, int sd,
+                                          const int* rot, double (*T)[DIM + 2]) {
+  constexpr int npl = line_nodes(NQ, DIM);
+#pragma unroll
+  for (int m = 0; m < NQ; ++m) {
+    const int n = base + m * sd;
+    double f[DIM + 2];
+    f[0] = sq[(1 + rot[0]) * npl + n];
+    const double un = __dmul_rn(f[0], sx[n]);
+    f[1] = fma(f[0], un, sx[npl + n]);
+#pragma unroll
+    for (int c = 1; c < DIM; ++c) f[1 + c] = __dmul_rn(sq[(1 + rot[c]) * npl + n], un);
+    f[DIM + 1] = __dmul_rn(sx[2 * npl + n], un);
+#pragma unroll
+    for (int a = 0; a < NQ; ++a)
+#pragma unroll
+      for (int s = 0; s < DIM + 2; ++s) T[a][s] = fma(A.cfd[a * NQ + m], f[s], T[a][s]);
   }
 }
 
@@ -615,6 +644,11 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
                 uu += uf * uf;
               }
               sf[DIM * NPL] = (VK == VK_EC32) ? uu : (float)q[r][DIM + 1] * rinvf;
+            } else if constexpr (VK == VK_WEAK) {
+              sx[0] = rinv;
+              sx[NPL] = L.pde ? p - __ldg(A.aux + (DIM + 2) * A.stride + g0 + v) : p;
+              sx[2 * NPL] = q[r][DIM + 1] + p;
+              sx[(S::ND - 1) * NPL] = 0.25 * a0;
             } else {
 #pragma unroll
               for (int c = 0; c < DIM; ++c) sx[c * NPL] = 0.5 * u[c];
@@ -681,7 +715,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
 #pragma unroll
         for (int k = 0; k < NAM; ++k) apv[k] = 0.0;
         apv[0] = ap[i];
-        if (LAW == LAW_EG && A.naux_nl > 1) {
+        if (LAW == LAW_EG && (RUS ? L.pde != 0 : A.naux_nl > 1)) {
           const size_t mid = (size_t)e * NP + line_base<NQ, DIM>(d, l, NQ) +
                              (size_t)(i ? (NQ - 1) : 0) * line_stride<NQ, DIM>(d, NQ);
 #pragma unroll
@@ -839,8 +873,10 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         form = near ? 0 : rmax < 3.0 * rmin && bmax < 3.0 * bmin ? 1 : 2;
     }
     if (act) {
-      // ---- two-point fluxes of the line's pairs
-      if constexpr (VK == VK_EC && !S::SW) {
+      // ---- two-point fluxes of the line's pairs, or the weak form's rows
+      if constexpr (VK == VK_WEAK) {
+        line_weak<DIM, NQ>(A, sq, sx, base, sd, rot, T);
+      } else if constexpr (VK == VK_EC && !S::SW) {
         const double c0 = 2.0 / (L.gamma - 1.0);
         if (form == 0)
           line_pairs<LAW, DIM, VK, NQ, 0>(A, c0, sq, sx, base, sd, rot, d, T, X);
@@ -913,6 +949,16 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     constexpr int NIN = FUSE ? 2 : 1;
     double in[RN][NIN][NS], gp[RN][DIM];
     {
+      if constexpr (VK == VK_WEAK) {
+#pragma unroll
+        for (int r = 0; r < RN; ++r) {
+          const unsigned v = tid + r * nth;
+          if (v < ne * NP) {
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) gp[r][k] = __ldg(A.aux + (1 + k) * A.stride + g0 + v);
+          }
+        }
+      }
       const bool rd = FUSE || epi == EPI_ADD || (epi == EPI_LSRK && A.a != 0.0) || epi == EPI_SUBOUT2 || epi == EPI_RLSRK;
       const bool o2 = epi == EPI_SUBOUT2 || epi == EPI_RLSRK;
       if (rd) {
@@ -966,6 +1012,13 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         }
       };
       if (cor) coriolis(L.omega, T);
+      if constexpr (VK == VK_WEAK) {  // -rho grad Phi (the pair fluxes carry it otherwise)
+        if ((A.dirs >> DZ) & 1) {
+          const double rho = L.pde ? qn[0] - __ldg(A.aux + (DIM + 1) * A.stride + gid) : qn[0];
+#pragma unroll
+          for (int k = 0; k < DIM; ++k) T[1 + k] = fma(-rho, gp[r][k], T[1 + k]);
+        }
+      }
       if constexpr (FUSE) {
 #pragma unroll
         for (int s = 0; s < NS; ++s) TL[s] = qn[OT + s * NPL];

@@ -12,6 +12,8 @@ tend_launch_fn fd_eg3_ec32_any(int nq);
 tend_launch_fn fd_eg3_kg_rus(int nq);
 tend_launch_fn fd_eg3_kg_any(int nq);
 tend_launch_fn fd_eg3_kg32_any(int nq);
+tend_launch_fn fd_eg3_weak_rus(int nq);
+tend_launch_fn fd_eg3_weak_any(int nq);
 tend_launch_fn fd_eg3_ec_fused_rus(int nq);
 tend_launch_fn fd_eg3_ec_fused_any(int nq);
 tend_launch_fn fd_eg3_ec32_fused_rus(int nq);
@@ -40,6 +42,7 @@ tend_launch_fn pick_fd(int law, int dim, int vk, int nq, int sflux) {
     if (vk == VK_EC32) return rus ? fd_eg3_ec32_rus(nq) : fd_eg3_ec32_any(nq);
     if (vk == VK_KG) return rus ? fd_eg3_kg_rus(nq) : fd_eg3_kg_any(nq);
     if (vk == VK_KG32) return fd_eg3_kg32_any(nq);
+    if (vk == VK_WEAK) return rus ? fd_eg3_weak_rus(nq) : fd_eg3_weak_any(nq);
   }
   if (law == LAW_EG && dim == 2) {
     if (vk == VK_EC) return fd_eg2_ec_any(nq);
