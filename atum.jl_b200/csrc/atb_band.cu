@@ -9,9 +9,9 @@
 // formed on the fly as each row is reached (src/odesolvers.jl:346-349), so
 // Qhat never exists in memory.  Kernels, in the order launch_band_solve
 // prefers them:
-//   band_solve_warp_kernel   block recurrence on the FP64 matrix unit, one
-//                            warp per 8 lines, nonzero tiles only (ARK stages
-//                            whose right-hand side is given whole)
+//   band_solve_warp_kernel   block recurrence on the FP64 matrix unit, one or
+//                            two warps per 8 lines, nonzero tiles only (ARK
+//                            stages whose right-hand side is given whole)
 //   band_solve_mma_kernel    the same over dense blocks, one warp per 8 rows
 //   band_solve_rows_kernel   one-state laws
 //   band_solve_shared_kernel substitution over the shared factor (below)
@@ -27,6 +27,7 @@
 // ev+1 overlaps the arithmetic of element ev, and read back as warp broadcasts.
 #include "atb_generic.cuh"
 
+#include <cstdint>
 #include <cstdlib>
 #include <type_traits>
 #include <utility>
@@ -600,9 +601,13 @@ void mma_launch(const BandSolve& B, cudaStream_t st) {
 
 // ---------------------------------------------- warp-owned block recurrence
 // The same recurrence (y_e = Li_e b_e - G_e y_e-1, x_e = Ui_e y_e - H_e x_e+1)
-// with one warp per 8 lines computing EVERY row of the block: the element-to-
-// element dependency stays inside the warp, so the sequential chain carries
-// no CTA barrier.  The blocks' zero structure is exploited tile by tile:
+// with H warps per 8 lines, each computing 1/H of the block's row tiles; the
+// barrier that hands over the shared tiles also hands the previous element's
+// result from warp to warp.  A chain of KV elements leaves a lone warp waiting
+// most of the time, so few lines take H = 2; with more than four groups of 8
+// lines per SM, H = 1 has enough warps and fewer operand loads.  Measured on
+// B200: 234 groups of 11 elements at N = 3, 17.8 us with H = 1, 15.6 with 2;
+// 800 groups of 16 at N = 4, 35.8 and 37.3.  The blocks' zero structure is exploited tile by tile:
 // Li is lower and Ui upper triangular, and since DG elements couple only
 // through their face nodes, L_e,e-1 (U_e,e+1) is nonzero only in the last
 // (first) Ns columns, so G_e (H_e) is too -- the product with the previous
@@ -650,8 +655,21 @@ struct WarpSolveShape {
   static constexpr int T0 = pass_tiles(BW1, NS, 0), T1 = pass_tiles(BW1, NS, 1);
   static constexpr int FR = 32 * (T0 > T1 ? T0 : T1);     // doubles of one ring slot
   static constexpr int RS = 3;                            // ring depth (elements in flight)
-  static constexpr int WBUF = RS * KP * LD + 2 * RW * LD;  // per warp: RHS ring + 2 result buffers
+  static constexpr int WBUF = RS * KP * LD + 2 * RW * LD;  // per 8 lines: RHS ring + 2 result buffers
 };
+// which of H warps owns a row tile: tiles ranked by their count of nonzero
+// tiles (longest last in pass 0, first in pass 1), dealt 0 1 1 0
+__host__ __device__ constexpr int tile_owner(int H, int MT, int pass, int mt) {
+  const int r = (pass == 0 ? MT - 1 - mt : mt) & 3;
+  return H == 2 && (r == 1 || r == 2) ? 1 : 0;
+}
+// its position among the owner's
+__host__ __device__ constexpr int tile_slot(int H, int MT, int pass, int mt) {
+  int n = 0;
+  for (int m = 0; m < mt; ++m)
+    if (tile_owner(H, MT, pass, m) == tile_owner(H, MT, pass, mt)) ++n;
+  return n;
+}
 
 // frag[(e * (T0 + T1) + pass * T0 + tile_off(pass, mat, mt) + kt - lo) * 32 + lane]
 //   = M[8 mt + lane / 4][4 kt + lane % 4]   (zero outside BW1 x BW1)
@@ -705,25 +723,26 @@ __device__ __forceinline__ void cp_async16g(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
-template <int NQ, int NS, int NW>
-__global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolve B) {
+template <int NQ, int NS, int NW, int H>
+__global__ void __launch_bounds__(32 * NW * H) band_solve_warp_kernel(const BandSolve B) {
   constexpr int BW1 = NQ * NS;
   using S = WarpSolveShape<BW1, NS>;
   constexpr int MT = S::MT, KT = S::KT, KP = S::KP, RW = S::RW, LD = S::LD, FR = S::FR, RS = S::RS;
   constexpr int T0 = S::T0, T1 = S::T1;
-  constexpr int JT = (BW1 + 3) / 4;  // RHS rows per lane per element (4 rows x 8 lines per pass)
+  constexpr int JT = (BW1 + 4 * H - 1) / (4 * H);  // RHS rows per lane per element (4 rows x 8 lines per warp and pass)
   extern __shared__ __align__(16) double sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = H == 1 ? warp : warp / H, h = H == 1 ? 0 : warp % H;  // group of 8 lines, part of its row tiles
   const int g = lane >> 2, tq = lane & 3;
   double* Fr = sm;                                   // [RS][FR], shared by the CTA's warps
-  double* ring = sm + RS * FR + warp * S::WBUF;      // [RS][KP][LD]: right-hand sides
+  double* ring = sm + RS * FR + grp * S::WBUF;       // [RS][KP][LD]: right-hand sides
   double* Wb = ring + RS * KP * LD;                  // [2][RW][LD]: results of the last two elements
   const LineMap& M = B.M;
   const int KV = M.KV, nh = M.nh, Np = M.Np;
   const size_t lstep = (size_t)M.estep * Np;
-  const int line0 = (blockIdx.x * NW + warp) * 8;
-  for (int i = lane; i < S::WBUF; i += 32) ring[i] = 0.0;
-  // ---- RHS loader: lane owns line (lane & 7) and rows 4j + (lane >> 3)
+  const int line0 = (blockIdx.x * NW + grp) * 8;
+  for (int i = 32 * h + lane; i < S::WBUF; i += 32 * H) ring[i] = 0.0;
+  // ---- RHS loader: lane owns line (lane & 7) and rows 4 (H j + h) + (lane >> 3)
   const int ll = lane & 7;
   const bool lact = line0 + ll < M.nlines;
   const size_t lb = lact ? (size_t)M.e0[line0 + ll] * Np + (line0 + ll) % nh : 0;
@@ -731,7 +750,7 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
   int rsel[JT];
 #pragma unroll
   for (int j = 0; j < JT; ++j) {
-    const int row = 4 * j + (lane >> 3);
+    const int row = 4 * (H * j + h) + (lane >> 3);
     rsel[j] = (lact && row < BW1) ? row % NS : -1;
     roff[j] = lb + (row < BW1 ? (size_t)nh * (row / NS) : 0);
   }
@@ -745,19 +764,27 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
   const double* src[JT];
 #pragma unroll
   for (int j = 0; j < JT; ++j) src[j] = field(B.q, rsel[j] < 0 ? 0 : rsel[j]) + roff[j];
-  // ---- outputs: rows 8 mt + g, lines 2 tq + i (null: padding row or no line)
-  double* dst[MT][2];
+  // ---- outputs of the warp's row tiles: rows 8 mt + g, lines 2 tq + i (null:
+  // padding row or no line)
+  constexpr int MTH = H == 1 ? MT : (MT + 2) / 2;  // row tiles of one warp, at most
+  double* dst[MTH][2];
+  auto set_dst = [&](auto passc) {
+    constexpr int P = decltype(passc)::value;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int line = line0 + 2 * tq + i;
-    const bool act = line < M.nlines;
-    const size_t ob = act ? (size_t)M.e0[line] * Np + line % nh : 0;
+    for (int i = 0; i < 2; ++i) {
+      const int line = line0 + 2 * tq + i;
+      const bool act = line < M.nlines;
+      const size_t ob = act ? (size_t)M.e0[line] * Np + line % nh : 0;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const int row = 8 * mt + g;
-      dst[mt][i] = (act && row < BW1) ? field(B.out, row % NS) + (size_t)nh * (row / NS) + ob : nullptr;
+      for (int mt = 0; mt < MT; ++mt) {
+        const int row = 8 * mt + g;
+        if (h == tile_owner(H, MT, P, mt))
+          dst[tile_slot(H, MT, P, mt)][i] =
+              (act && row < BW1) ? field(B.out, row % NS) + (size_t)nh * (row / NS) + ob : nullptr;
+      }
     }
-  }
+  };
+  set_dst(std::integral_constant<int, 0>{});
   // element ev of pass P (its tiles and this warp's RHS) into ring slot
   // ev % RS; evoff = ev * (element step in the fields)
   auto issue = [&](auto passc, int ev, int slot, size_t evoff) {
@@ -767,17 +794,17 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
       const double* gf = B.frag + ((size_t)ev * (T0 + T1) + (P ? T0 : 0)) * 32 + 2 * threadIdx.x;
       double* sf = Fr + slot * FR + 2 * threadIdx.x;
 #pragma unroll
-      for (int c = 0; c < n16; c += 32 * NW)
+      for (int c = 0; c < n16; c += 32 * NW * H)
         if (c + (int)threadIdx.x < n16) cp_async16g(sf + 2 * c, gf + 2 * c);
-      double* sr = ring + slot * KP * LD + (lane >> 3) * LD + ll;
+      double* sr = ring + slot * KP * LD + (4 * h + (lane >> 3)) * LD + ll;
 #pragma unroll
       for (int j = 0; j < JT; ++j)
-        if (rsel[j] >= 0) cp_async8(sr + 4 * j * LD, src[j] + evoff);
+        if (rsel[j] >= 0) cp_async8(sr + 4 * H * j * LD, src[j] + evoff);
     }
     cp_async_commit();
   };
-  auto step = [&](auto passc, int slot, size_t evoff, int par) {
-    constexpr int P = decltype(passc)::value;
+  auto half_step = [&](auto passc, auto hc, int slot, size_t evoff, int par) {
+    constexpr int P = decltype(passc)::value, HH = decltype(hc)::value;
     const double* F = Fr + slot * FR + lane;
     const double* V = ring + slot * KP * LD;
     const double* Wp = Wb + (par ^ 1) * RW * LD;
@@ -804,7 +831,7 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
       static_for<MT>([&](auto mtc) {
         constexpr int mt = decltype(mtc)::value;
         constexpr TileRange rc = tile_range(BW1, NS, P, 1, mt);
-        if constexpr (kt >= rc.lo && kt <= rc.hi) {
+        if constexpr (tile_owner(H, MT, P, mt) == HH && kt >= rc.lo && kt <= rc.hi) {
           constexpr int off = (tile_off(BW1, NS, P, 1, mt) + kt - rc.lo) * 32;
           dmma_8x8x4(aC[mt][0], aC[mt][1], F[off], bw[kt]);
         }
@@ -815,7 +842,7 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
       static_for<MT>([&](auto mtc) {
         constexpr int mt = decltype(mtc)::value;
         constexpr TileRange ra = tile_range(BW1, NS, P, 0, mt);
-        if constexpr (kt >= ra.lo && kt <= ra.hi) {
+        if constexpr (tile_owner(H, MT, P, mt) == HH && kt >= ra.lo && kt <= ra.hi) {
           constexpr int off = (tile_off(BW1, NS, P, 0, mt) + kt - ra.lo) * 32;
           dmma_8x8x4(aA[mt][0], aA[mt][1], F[off], bv[kt]);
         }
@@ -823,11 +850,23 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
     });
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
+      if (tile_owner(H, MT, P, mt) != HH) continue;
+      const int k = tile_slot(H, MT, P, mt);
       const int row = 8 * mt + g;
       const double y0 = aA[mt][0] + aC[mt][0], y1 = aA[mt][1] + aC[mt][1];
       *reinterpret_cast<double2*>(Wn + row * LD + 2 * tq) = make_double2(y0, y1);
-      if (dst[mt][0]) dst[mt][0][evoff] = y0;
-      if (dst[mt][1]) dst[mt][1][evoff] = y1;
+      if (dst[k][0]) dst[k][0][evoff] = y0;
+      if (dst[k][1]) dst[k][1][evoff] = y1;
+    }
+  };
+  auto step = [&](auto passc, int slot, size_t evoff, int par) {
+    if constexpr (H == 1) {
+      half_step(passc, std::integral_constant<int, 0>{}, slot, evoff, par);
+    } else {
+      if (h == 0)
+        half_step(passc, std::integral_constant<int, 0>{}, slot, evoff, par);
+      else
+        half_step(passc, std::integral_constant<int, 1>{}, slot, evoff, par);
     }
   };
   const std::integral_constant<int, 0> fwd{};
@@ -859,7 +898,8 @@ __global__ void __launch_bounds__(32 * NW) band_solve_warp_kernel(const BandSolv
 #pragma unroll
   for (int j = 0; j < JT; ++j) src[j] = field(B.out, rsel[j] < 0 ? 0 : rsel[j]) + roff[j];
   // x_KV = 0: the buffer read first holds zeros
-  for (int i = lane; i < RW * LD; i += 32) Wb[((KV & 1) ^ 1) * RW * LD + i] = 0.0;
+  for (int i = 32 * h + lane; i < RW * LD; i += 32 * H) Wb[((KV & 1) ^ 1) * RW * LD + i] = 0.0;
+  if constexpr (H > 1) set_dst(bwd);  // (the same tiles with one warp)
   // slot: (KV - 1 - ev) % RS, i.e. the step count t % RS
   issue(bwd, KV - 1, 0, (size_t)(KV - 1) * lstep);
   issue(bwd, KV - 2, 1, (size_t)(KV - 2) * lstep);
@@ -889,22 +929,23 @@ constexpr size_t warp_solve_smem() {
 
 constexpr size_t kWarpSolveSmemMax = 227 * 1024;
 
-template <int NQ, int NS, int NW>
+template <int NQ, int NS, int NW, int H>
 void warp_launch_nw(const BandSolve& B, cudaStream_t st) {
   constexpr size_t smem = warp_solve_smem<NQ, NS, NW>();
   static bool configured = false;
   if (!configured && smem > 48 * 1024)
-    cudaFuncSetAttribute(band_solve_warp_kernel<NQ, NS, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(band_solve_warp_kernel<NQ, NS, NW, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   configured = true;
   const int warps = (B.M.nlines + 7) / 8;
-  launch_maybe_pdl(band_solve_warp_kernel<NQ, NS, NW>, dim3((warps + NW - 1) / NW), dim3(32 * NW), smem, st, B);
+  launch_maybe_pdl(band_solve_warp_kernel<NQ, NS, NW, H>, dim3((warps + NW - 1) / NW),
+                   dim3(32 * NW * H), smem, st, B);
 }
 
-// Warps per CTA: the element steps are bound by the issue rate of each SM, so
-// the time goes with the warps the busiest SM runs in total, ceil(CTAs / SMs)
-// x NW; among counts within 2% of each other, CTAs on every SM, then more
-// warps resident at once (latency hiding), then more warps per CTA (each copy
-// of the tiles shared by more lines).
+// Groups of 8 lines per CTA: the element steps are bound by the matrix unit and
+// issue rate of each SM, so the time goes with the groups the busiest SM runs
+// in total, ceil(CTAs / SMs) x NW; among counts within 2% of each other, CTAs on
+// every SM, then more groups resident at once (latency hiding), then more
+// groups per CTA (each copy of the tiles shared by more lines).
 inline int pick_nw(int warps, int nsm, const size_t smem[4]) {
   static const int cand[4] = {2, 3, 4, 6};
   int best = -1;
@@ -944,11 +985,21 @@ bool warp_launch(const BandSolve& B, cudaStream_t st) {
   }
   const size_t smem[4] = {warp_solve_smem<NQ, NS, 2>(), warp_solve_smem<NQ, NS, 3>(), warp_solve_smem<NQ, NS, 4>(),
                           warp_solve_smem<NQ, NS, 6>()};
-  switch (pick_nw((B.M.nlines + 7) / 8, nsm, smem)) {
-    case 2: warp_launch_nw<NQ, NS, 2>(B, st); return true;
-    case 3: warp_launch_nw<NQ, NS, 3>(B, st); return true;
-    case 4: warp_launch_nw<NQ, NS, 4>(B, st); return true;
-    case 6: warp_launch_nw<NQ, NS, 6>(B, st); return true;
+  const int groups = (B.M.nlines + 7) / 8;
+  if constexpr (WarpSolveShape<NQ * NS, NS>::MT > 1) {
+    if (groups <= 4 * nsm) {  // few lines: two warps per group (measured above)
+      const size_t two[4] = {smem[0], smem[1], SIZE_MAX, SIZE_MAX};
+      switch (pick_nw(groups, nsm, two)) {
+        case 2: warp_launch_nw<NQ, NS, 2, 2>(B, st); return true;
+        case 3: warp_launch_nw<NQ, NS, 3, 2>(B, st); return true;
+      }
+    }
+  }
+  switch (pick_nw(groups, nsm, smem)) {
+    case 2: warp_launch_nw<NQ, NS, 2, 1>(B, st); return true;
+    case 3: warp_launch_nw<NQ, NS, 3, 1>(B, st); return true;
+    case 4: warp_launch_nw<NQ, NS, 4, 1>(B, st); return true;
+    case 6: warp_launch_nw<NQ, NS, 6, 1>(B, st); return true;
   }
   return false;
 }
