@@ -449,11 +449,11 @@ def run_ours(args):
                 "steps": ke},
         "gpu_launches": int(n1.value - n0.value),
         "roofline": {"bound": "fp64",
-                     "kernel": ("tendency_kernel<EulerGravity,3,EC,Nq=5,fused> (ARK23 stage: EC tendency + linear "
+                     "kernel": ("fd_kernel<EulerGravity,3,EC,Nq=5,fused> (ARK23 stage: EC tendency + linear "
                                 "vertical operator)") if fused else
-                               ("tendency_kernel<EulerGravity,3,EC,Nq=5> (LSRK54 stage: tendency + register "
+                               ("fd_kernel<EulerGravity,3,EC,Nq=5> (LSRK54 stage: tendency + register "
                                 "update)" if scheme == "lsrk54" else
-                                "tendency_kernel<EulerGravity,3,EC,Nq=5> (explicit stage tendency)"),
+                                "fd_kernel<EulerGravity,3,EC,Nq=5> (explicit stage tendency)"),
                      "flops_per_dof_stage": flops_dof,
                      "achieved": tflops, "peak": peak_fp64.value, "unit": "TFLOP/s",
                      "frac": tflops / peak_fp64.value if peak_fp64.value > 0 else None,
@@ -525,8 +525,8 @@ def precision_pair(A, args, scheme, value_fp64):
             "mass_drift_fp32flux": abs(float(np.sum(mj * hb[0])) - m0) / abs(m0)}
 
 
-PROFILE_TEND = "profiles/tendency_eg3_ec_nq5_bubble16.md"
-PROFILE_FUSED = "profiles/tendency_eg3_ec_nq5_fused_bubble16.md"
+PROFILE_TEND = None  # no capture of the line kernel without the fused operator
+PROFILE_FUSED = "profiles/fd_eg3_ec_nq5_fused_bubble16.md"
 
 
 # ------------------------------------------------------------ serving stream
@@ -807,7 +807,7 @@ def run_c5(args):
         avg = t["ms"] / max(1, t["launches"])
         fl = (FLOPS_PER_DOF_STAGE["bubble_3d_N7_ec_rusanov"] +
               (FLOPS_PER_DOF_STAGE["bubble_3d_N7_linear_weak_z"] if fused else 0.0)) * dofs
-        out["stage_kernel"] = {"kernel": "tendency_kernel<EulerGravity,3,%s,Nq=8%s>" %
+        out["stage_kernel"] = {"kernel": "fd_kernel<EulerGravity,3,%s,Nq=8%s>" %
                                ("EC" if precision == "fp64" else "EC32", ",fused" if fused else ""),
                                "avg_launch_ms": avg, "bound": "fp64", "achieved_tflops": fl / (avg * 1e-3) / 1e12,
                                "peak_tflops": peak_fp64.value,
@@ -961,8 +961,8 @@ def run_sphere(args):
     # operator and the ARK accumulation when the solver fuses them
     fused = prof["tendency_linear"]["launches"] == 0
     tend = kern("tendency", ["sphere_N5_ec_rusanov"] + (["sphere_N5_linear_weak_z"] if fused else []),
-                "curved_kernel<EulerGravity,EC,Rusanov,fused> (ARK23 stage: EC tendency + radial linear operator)"
-                if fused else "curved_kernel<EulerGravity,EC> (explicit stage tendency)")
+                "curved_fd_kernel<EulerGravity,EC,Rusanov,fused> (ARK23 stage: EC tendency + radial linear operator)"
+                if fused else "curved_fd_kernel<EulerGravity,EC> (explicit stage tendency)")
     lin = kern("tendency_linear", ["sphere_N5_linear_weak_z"],
                "curved_kernel<LinearEulerGravity,WEAK> (vertical linear operator + ARK accumulation)")
     b = prof["band_solve"]
@@ -976,7 +976,7 @@ def run_sphere(args):
         nlines = 6 * KH * KH * (N + 1) ** 2
         BW1 = 5 * (N + 1)
         byt = (nlines * (KV * BW1 * BW1 + 2 * (KV - 1) * 25) + 4 * dofs) * 8
-        band = {"kernel": "band_solve_lines_kernel<6,5,sparse> (one factor per vertical line)", "avg_launch_ms": avgb,
+        band = {"kernel": "band_solve_stream_kernel<6,5> (one factor per vertical line)", "avg_launch_ms": avgb,
                 "bound": "hbm", "bytes_per_launch": byt, "achieved_gbs": byt / (avgb * 1e-3) / 1e9,
                 "peak_gbs": peaks["hbm_gbs"], "frac": byt / (avgb * 1e-3) / 1e9 / peaks["hbm_gbs"],
                 "peak_kind": kind}
@@ -1162,9 +1162,11 @@ def run_swbatch(args):
     return 0
 
 
-def profiled_traffic(profile=PROFILE_TEND):
+def profiled_traffic(profile):
     """DRAM bytes (read + write) of one FP64 launch of the kernel and workload
-    a committed ncu summary covers."""
+    a committed ncu summary covers (None: none does)."""
+    if profile is None:
+        return None
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), profile)
     try:
         with open(path) as f:
