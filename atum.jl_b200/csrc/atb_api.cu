@@ -144,6 +144,7 @@ struct atb_op {
   int ninst = 1;      // instances packed into this operator
   int K_active = 0;   // elements the tendency launches cover (a prefix of K)
   int device = -1;    // the CUDA device current at creation (its memory holds every buffer)
+  int nsm = 0;        // its multiprocessors
   std::vector<int> inst_off;  // first element of each instance, then K
   std::vector<int> col_e0;    // bottom element of every vertical column
   bool cols_uniform = true;   // every instance has the same element counts
@@ -538,8 +539,14 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
     cudaGetLastError();
     return fail(ATB_ERR_CUDA, "no usable CUDA device");
   }
+  int nsm = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) {
+    cudaGetLastError();
+    return fail(ATB_ERR_CUDA, "no multiprocessor count for the current device");
+  }
   atb_op* op = new atb_op();
   op->device = dev;
+  op->nsm = nsm;
   op->launch = fn;
   op->reducer = rf;
   op->dim = d->dim;
@@ -628,7 +635,7 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
     op->fd = true;
     // Cfd, or Cw for the weak form
     std::copy_n(tab.begin() + (vk == VK_WEAK ? Nq * Nq : 0), Nq * Nq, op->cfd);
-    op->E = fd_default_elements(line_count(Nq, dim), fd_limit(op), K);
+    op->E = fd_default_elements(Nq, dim, fd_limit(op), K, nsm, false);
   }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
@@ -753,7 +760,7 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
   if (d->law == LAW_EG) nu = d->pde_level_balance ? 6 : (op->vk == VK_WEAK ? 4 : 1);
   if (d->law == LAW_LEG) nu = 6;
   op->naux_used = std::min(nu, op->naux);
-  op->E = fd ? fd_default_elements(line_count(Nq, 3), fd_limit(op), K) : std::max(1, 128 / Np);
+  op->E = fd ? fd_default_elements(Nq, 3, fd_limit(op), K, op->nsm, true) : std::max(1, 128 / Np);
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
   if (op->smem > 227 * 1024 || (!fd && cta_threads(op->E, Np) > 512)) {

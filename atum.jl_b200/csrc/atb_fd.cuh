@@ -109,8 +109,15 @@ inline int fd_max_elements(int law, int dim, int vk, int nq) {
 }
 // Elements per CTA when nothing else asks for a count: the fullest last warp
 // among CTAs of at least 96 threads (the smallest such), but no fewer CTAs than
-// SMs where the operator has the elements for it.
-inline int fd_default_elements(int nl, int emax, int K) {
+// SMs where the operator has the elements for it.  While every element's warps
+// can have a scheduler to themselves, one element: the pairs take as long as in
+// a full warp and the other lanes share the staging (2-D Euler-gravity N = 7,
+// 24x24 elements: 10.2 us per LSRK54 stage at 4 elements, 9.0 at 1; 3-D N = 3,
+// 6^3: 4.1 at 2, 3.6 at 1); not below 16 lines an element, where it measured
+// within 4 % either way, nor on curved elements (162 at N = 4: 8.4 us at 2, 8.9 at 1).
+inline int fd_default_elements(int nq, int dim, int emax, int K, int nsm, bool curved) {
+  const int nl = line_count(nq, dim);
+  if (!curved && nq >= 4 && nl >= 16 && (long long)K * ((nl + 31) / 32) <= 4LL * nsm) return 1;
   int best = emax;
   double fill = 0.0;
   for (int E = 1; E <= emax; ++E) {
@@ -119,7 +126,7 @@ inline int fd_default_elements(int nl, int emax, int K) {
     const double f = (double)(E * nl) / th;
     if (f > fill + 1e-9) { fill = f; best = E; }
   }
-  const int spread = (K + 147) / 148;
+  const int spread = (K + nsm - 1) / nsm;
   return best < spread ? best : spread < 1 ? 1 : spread;
 }
 inline int fd_threads(int nq, int dim, int E) { return ((E * line_count(nq, dim) + 31) / 32) * 32; }
@@ -421,11 +428,12 @@ __device__ __forceinline__ void line_flux_dir(const LawP& L, int kind, bool f32,
   if (!f32 || !surface_flux32<LAW, DIM>(L, kind, 0, sgn, qm, am, qp, ap, nf))
     surface_flux<LAW, DIM>(L, kind, 0, sgn, qm, am, qp, ap, nf);
 }
-// every flux in either precision form, chosen at run time: one out-of-line copy
-template <int LAW, int DIM>
-__device__ __noinline__ void line_flux_any(const LawP& L, int kind, bool f32, double sgn, const double* qm,
-                                           const double* am, const double* qp, const double* ap, double* nf) {
-  line_flux_dir<LAW, DIM>(L, kind, f32, sgn, qm, am, qp, ap, nf);
+// every flux, chosen at run time: one out-of-line copy for each precision form (one
+// for both cost the FP64 operators 1 to 5 %)
+template <int LAW, int DIM, bool F32>
+__device__ __noinline__ void line_flux_any(const LawP& L, int kind, double sgn, const double* qm, const double* am,
+                                           const double* qp, const double* ap, double* nf) {
+  line_flux_dir<LAW, DIM>(L, kind, F32, sgn, qm, am, qp, ap, nf);
 }
 
 // rotated component c of direction d: the normal component first
@@ -662,8 +670,10 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           line_rusanov<LAW, DIM>(L, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
         else if constexpr (SF >= 0)
           line_flux_dir<LAW, DIM>(L, SF, S::F32, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
+        else if (S::F32 || (!S::SW && A.sf32))
+          line_flux_any<LAW, DIM, true>(L, sflux, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
         else
-          line_flux_any<LAW, DIM>(L, sflux, A.sf32, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
+          line_flux_any<LAW, DIM, false>(L, sflux, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {

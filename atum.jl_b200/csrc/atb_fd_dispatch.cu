@@ -16,6 +16,7 @@ tend_launch_fn fd_eg3_ec_fused_any(int nq);
 tend_launch_fn fd_euler3_ec_any(int nq);
 tend_launch_fn fd_euler2_ec_rus(int nq);
 tend_launch_fn fd_euler2_ec_any(int nq);
+tend_launch_fn fd_eg2_ec_rus(int nq);
 tend_launch_fn fd_eg2_ec_any(int nq);
 tend_launch_fn fd_sw2_ec_rus(int nq);
 tend_launch_fn fd_sw2_ec32_rus(int nq);
@@ -47,7 +48,7 @@ tend_launch_fn pick_fd(int law, int dim, int vk, int nq, int sflux) {
     if (vk == VK_KG) return rus ? fd_eg3_kg_rus(nq) : fd_eg3_kg_any(nq);
     if (vk == VK_WEAK) return rus ? fd_eg3_weak_rus(nq) : fd_eg3_weak_any(nq);
   }
-  if (law == LAW_EG && dim == 2 && vk == VK_EC) return fd_eg2_ec_any(nq);
+  if (law == LAW_EG && dim == 2 && vk == VK_EC) return rus ? fd_eg2_ec_rus(nq) : fd_eg2_ec_any(nq);
   if (law == LAW_EULER && dim == 3 && vk == VK_EC) return fd_euler3_ec_any(nq);
   if (law == LAW_EULER && dim == 2 && vk == VK_EC) return rus ? fd_euler2_ec_rus(nq) : fd_euler2_ec_any(nq);
   if (law == LAW_SW && dim == 2) {
