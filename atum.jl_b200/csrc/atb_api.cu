@@ -138,7 +138,6 @@ struct atb_op {
   LawP law{};
   int dim = 0, N = 0, Nq = 0, Np = 0, Nfp = 0, K = 0, Kd[3] = {1, 1, 1}, ns = 0, naux = 0;
   int vk = 0, dirs = 0, sflux = 0, precision = 0, stacked = 0;
-  int fvk = 0;  // the volume kind its line kernel runs (fd_volume_kind)
   int naux_used = 0;  // leading aux components the tendency kernel stages
   atb_op_desc kind{};  // instance 0's descriptor (kind checks of later placements)
   int ninst = 1;      // instances packed into this operator
@@ -205,10 +204,10 @@ size_t node_smem(const atb_op* op, int E) {
 // the line-per-thread kernels (brick or curved elements): most elements per CTA
 // they are compiled for, shared memory
 int fd_limit(const atb_op* op) {
-  return op->curved ? curved_fd_elements(op->Nq) : fd_max_elements(op->law.kind, op->dim, op->fvk, op->Nq);
+  return op->curved ? curved_fd_elements(op->Nq) : fd_max_elements(op->law.kind, op->dim, op->vk, op->Nq);
 }
 size_t fd_bytes(const atb_op* op, int E, bool fuse) {
-  return op->curved ? curved_fd_smem_bytes(op->Nq, E, fuse) : fd_smem_bytes(op->law.kind, op->dim, op->fvk, op->Nq, E, fuse);
+  return op->curved ? curved_fd_smem_bytes(op->Nq, E, fuse) : fd_smem_bytes(op->law.kind, op->dim, op->vk, op->Nq, E, fuse);
 }
 // elements and threads of a tendency launch (the shape does not change results)
 int op_elements(const atb_op* op) { return op->fd ? std::min(op->E, fd_limit(op)) : op->E; }
@@ -235,7 +234,6 @@ void fill_args(const atb_op* op, TendArgs& A) {
   A.law = op->law;
   A.dirs = op->dirs;
   A.sflux = op->sflux;
-  A.sf32 = op->precision == ATB_PREC_FP32FLUX;
   A.stride = op->stride();
   A.a = 0;
   A.bdt = 0;
@@ -573,7 +571,6 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
   op->ns = (d->law == LAW_ADV) ? 1 : d->dim + 2;
   op->naux = d->naux;
   op->vk = vk;
-  op->fvk = fd_volume_kind(d->law, vk);
   op->dirs = d->directions;
   op->sflux = sf;
   op->precision = d->precision;
@@ -1503,7 +1500,7 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
   int E = op_elements(op);
   auto bytes = [&](int e) { return fd_bytes(op, e, true); };
   const size_t share =
-      op->curved ? 227 * 1024 / 2 - 1024 : 227 * 1024 / fd_cfg(op->law.kind, op->dim, op->fvk, op->Nq).min_blocks - 1024;
+      op->curved ? 227 * 1024 / 2 - 1024 : 227 * 1024 / fd_cfg(op->law.kind, op->dim, op->vk, op->Nq).min_blocks - 1024;
   while (E > 1 && bytes(E) > share) --E;
   A.E = E;
   A.epi = EPI_ARK;

@@ -24,12 +24,9 @@
 //
 // Direction-agnostic code: a thread reads the velocity (momentum) components
 // rotated so that its line's normal component comes first, so one instruction
-// stream serves all directions, lanes of one warp included.
-//
-// The FP32-flux forms of Euler and Euler-gravity have no kernel here: the FP64
-// one serves them (atb_fd_dispatch.cu), with the surface fluxes that are chosen at
-// run time in FP32 (2-D Euler 24x24 elements N = 7, Roe: 10.1 us per LSRK54 stage,
-// 11.2 with FP64 surface fluxes).
+// stream serves all directions, lanes of one warp included.  The FP32-flux
+// entropy-conservative flux keeps the components in x, y, z order and selects
+// (its FP32 sums then round as they always did).
 //
 // Shared memory per element: state (NS), point values (NX), all in rows of
 // Nq | 1 doubles (an odd row stride keeps x-lines free of bank conflicts); the
@@ -58,7 +55,7 @@ template <int LAW, int DIM, int VK> struct LineShape {
   static constexpr int NS = NSt<LAW, DIM>::v;
   static constexpr bool EG = LAW == LAW_EG;
   static constexpr bool SW = LAW == LAW_SW;
-  static constexpr bool F32 = VK == VK_EC32;  // (shallow water only)
+  static constexpr bool F32 = VK == VK_EC32 || VK == VK_KG32;
   // a third quantity per node pair, contracted like the flux and scaled by a
   // node value at the end: the gravity fluctuation (EG) or the bathymetry
   // difference (shallow water)
@@ -66,10 +63,15 @@ template <int LAW, int DIM, int VK> struct LineShape {
   // point values per node, in doubles:
   //   EC (Euler, EG)  u/2 (DIM), B = rho/p, p/rho [, Phi/4]
   //   KG              u/2 (DIM), p/2, e/2 [, Phi/4]
+  //   EC32            p, b = rho/2p, p/rho [, Phi], then FP32 u (DIM), |u|^2
+  //   KG32            p [, Phi], then FP32 u (DIM), e
   //   WEAK (EG)       1/rho, p (less the reference), rho e + p, Phi/4
   //   EC (SW)         u/2 (DIM), theta/2, b
   //   EC32 (SW)       b, then FP32 u (DIM), theta
-  static constexpr int ND = (VK == VK_WEAK) ? 4 : F32 ? 1 : DIM + 2 + (EG ? 1 : 0);
+  static constexpr int ND = VK == VK_WEAK ? 4
+                               : SW ? (F32 ? 1 : DIM + 2)
+                               : (VK == VK_EC32) ? 3 + (EG ? 1 : 0) : (VK == VK_KG32) ? 1 + (EG ? 1 : 0)
+                                                                                       : DIM + 2 + (EG ? 1 : 0);
   static constexpr int NF = F32 ? DIM + 1 : 0;  // FP32 values
   static constexpr int NX = ND + (NF + 1) / 2;
   // the accumulators (NS per node) reuse the region of the point values
@@ -86,11 +88,13 @@ __host__ __device__ constexpr int line_nodes(int nq, int dim) { return line_row(
 // cost more (3-D, Nq = 6: 718 us per LSRK54 step of 20^3 elements at 4 CTAs of
 // 128 threads, 750 at 2 of 224; Nq = 5 fused stage: 44 us at 3 CTAs of 160
 // threads, 49 at 2, 74 at 4); one accumulator array pays where shared memory
-// limits the CTAs (shallow water, Nq = 5: 561 against 612 us).
+// or the FP32-flux form's registers limit the CTAs (shallow water, Nq = 5:
+// 561 against 612 us).
 struct FdCfg {
   int max_threads, min_blocks, bufs;
 };
 __host__ __device__ constexpr FdCfg fd_cfg(int law, int dim, int vk, int nq) {
+  const bool f32 = vk == VK_EC32 || vk == VK_KG32;
   if (dim == 2) return law == LAW_SW ? FdCfg{160, nq <= 5 ? 4 : 3, 1} : FdCfg{224, 2, 2};
   // weak form: little arithmetic, so more CTAs for the memory (24^3 elements, N =
   // 4: 75 us at 4 of 160 threads and one array, 82 at 3 and three arrays, 95 at
@@ -99,7 +103,7 @@ __host__ __device__ constexpr FdCfg fd_cfg(int law, int dim, int vk, int nq) {
   if (nq == 8) return FdCfg{192, 2, 1};
   if (nq == 7) return FdCfg{160, 3, 1};
   if (nq == 6) return FdCfg{128, 4, 1};
-  if (nq == 5) return FdCfg{160, 3, 3};
+  if (nq == 5 || f32) return FdCfg{160, 3, f32 ? 1 : 3};
   return FdCfg{224, 2, 3};
 }
 __host__ __device__ constexpr int line_count(int nq, int dim) { return dim * ipow(nq, dim - 1); }
@@ -138,7 +142,10 @@ __host__ __device__ constexpr int fd_slot(int ns, int nxa, int nq, int dim, int 
 }
 inline int fd_nx(int law, int dim, int vk) {
   const int ns = dim + 2;
-  const int nx = vk == VK_WEAK ? 4 : vk == VK_EC32 ? 1 + (dim + 2) / 2 : dim + 2 + (law == LAW_EG ? 1 : 0);
+  const bool f32 = vk == VK_EC32 || vk == VK_KG32;
+  const int eg = law == LAW_EG ? 1 : 0;
+  const int nd = vk == VK_WEAK ? 4 : law == LAW_SW ? (f32 ? 1 : dim + 2) : vk == VK_EC32 ? 3 + eg : vk == VK_KG32 ? 1 + eg : dim + 2 + eg;
+  const int nx = nd + (f32 ? (dim + 2) / 2 : 0);
   return nx > ns ? nx : ns;
 }
 inline size_t fd_smem_bytes(int law, int dim, int vk, int nq, int E, bool fuse) {
@@ -148,11 +155,12 @@ inline size_t fd_smem_bytes(int law, int dim, int vk, int nq, int E, bool fuse) 
 
 // ------------------------------------------------------------ pair fluxes
 // Point values of one node as a pair flux reads them; velocities rotated
-// (normal component first).
+// (normal component first) in the FP64 forms.
 template <int LAW, int DIM, int VK> struct LinePt {
   double r, v[DIM + 1], ph;     // EC: v = u/2 .., B; KG: u/2 .., e/2; SW: u/2 .., theta/2
   double w;                     // KG: p/2; SW: normal momentum / 2
-  float uf[DIM], xf;            // SW EC32: u, theta
+  double p, b;                  // EC32: p, b; KG32: p
+  float uf[DIM], xf;            // EC32: u, |u|^2; KG32: u, e; SW EC32: u, theta
 };
 
 // VOL: read again for every pair (volatile): at Nq >= 6 in 3-D the compiler
@@ -179,6 +187,14 @@ __device__ __forceinline__ void line_load(LinePt<LAW, DIM, VK>& P, const double*
       for (int c = 0; c < DIM; ++c) P.v[c] = sx[rot[c] * npl + n];
       P.v[DIM] = sx[DIM * npl + n];
     }
+  } else if constexpr (S::F32) {
+    P.p = sx[n];
+    if constexpr (VK == VK_EC32) P.b = sx[npl + n];
+    if constexpr (S::EG) P.ph = sx[(S::ND - 1) * npl + n];
+    const FPtr sf = (const float*)(sx_ + S::ND * npl);
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) P.uf[c] = sf[(VK == VK_KG32 ? rot[c] : c) * npl + n];
+    P.xf = sf[DIM * npl + n];
   } else {
 #pragma unroll
     for (int c = 0; c < DIM; ++c) P.v[c] = sx[rot[c] * npl + n];
@@ -192,8 +208,8 @@ __device__ __forceinline__ void line_load(LinePt<LAW, DIM, VK>& P, const double*
   }
 }
 
-// Symmetric two-point flux f (components rotated: normal momentum at 1) and the
-// extra value x, antisymmetric in the pair.
+// Symmetric two-point flux f (components rotated: normal momentum at 1, except
+// VK_EC32, x y z order) and the extra value x, antisymmetric in the pair.
 //   EC: rho_log, p_c = rho_avg / (2 b_avg), and the energy flux in the form
 //       f_rho (1/(2 (g-1) b_log) + Phi_avg + u1.u2 / 2) + p_c u_n
 //       (|u_avg|^2 - |u|^2_avg / 2 = u1.u2 / 2), with one reciprocal for every
@@ -202,9 +218,13 @@ __device__ __forceinline__ void line_load(LinePt<LAW, DIM, VK>& P, const double*
 //   TIER: the line's values lie within a factor 1.2 (0), within a factor 3 (1: a
 //   longer polynomial; the core of a vortex on a coarse grid), or further apart
 //   (2: logarithms).  The form depends on the line alone, so results do not
-//   depend on the launch shape.
+//   depend on the launch shape.  The FP32-flux form's two versions (0: every
+//   pair on the series branch; 2: a branch per pair) give the same values, so
+//   there a warp takes one for all its lines; in 2-D only the second is
+//   compiled (the first gains nothing on a large grid and the second copy of
+//   the unrolled pairs costs a small one a third of its step).
 template <int LAW, int DIM, int VK, int TIER>
-__device__ __forceinline__ void line_pair(const LawP& L, double c0, const LinePt<LAW, DIM, VK>& P,
+__device__ __forceinline__ void line_pair(const LawP& L, double c0, int d, const LinePt<LAW, DIM, VK>& P,
                                           const LinePt<LAW, DIM, VK>& Q, double* f, double& x) {
   using S = LineShape<LAW, DIM, VK>;
   if constexpr (S::SW && !S::F32) {
@@ -224,6 +244,16 @@ __device__ __forceinline__ void line_pair(const LawP& L, double c0, const LinePt
     f[1] += L.grav * P.r * Q.r * 0.5;
     f[DIM + 1] = (double)(mdf * (0.5f * (P.xf + Q.xf)));
     x = P.ph - Q.ph;
+  } else if constexpr (VK == VK_KG32) {
+    kg_vol32<DIM>(0, P.r, P.p, P.uf, P.xf, Q.r, Q.p, Q.uf, Q.xf, f);
+    if constexpr (S::EG) x = ((P.r + Q.r) / 2.0 / 2.0) * (P.ph - Q.ph);
+  } else if constexpr (VK == VK_EC32) {
+    // ec_vol32 with the direction given at run time (the FP32 sums stay in
+    // x, y, z order)
+    double xr;
+    ec_vol32<LAW, DIM, TIER == 0>((float)c0, d, P.r, P.p, P.b, P.uf, P.xf, S::EG ? P.ph : 0.0, Q.r, Q.p, Q.b, Q.uf, Q.xf,
+                       S::EG ? Q.ph : 0.0, f, &xr);
+    if constexpr (S::EG) x = xr * (P.ph - Q.ph);
   } else if constexpr (VK == VK_KG) {
     const double ravg = 0.5 * (P.r + Q.r);
     double ua[DIM];
@@ -288,9 +318,9 @@ __device__ __forceinline__ void line_pairs(const TendArgs& A, double c0, const d
       LinePt<LAW, DIM, VK> Q;
       line_load<LAW, DIM, VK, DIM == 3 && NQ >= 6>(Q, sq, sx, npl, base + b * sd, rot, d);
       double f[NS], x = 0.0;
-      line_pair<LAW, DIM, VK, TIER>(A.law, c0, P, Q, f, x);
+      line_pair<LAW, DIM, VK, TIER>(A.law, c0, d, P, Q, f, x);
       const double cab = A.cfd[a * NQ + b], cba = A.cfd[b * NQ + a];
-      if constexpr (S::EG && VK == VK_KG) {
+      if constexpr (S::EG && (VK == VK_KG || VK == VK_KG32)) {
         // the fluctuation has no node factor: into the flux, as it cancels there
         const double fb = f[1] + x;
         f[1] = f[1] - x;
@@ -421,19 +451,42 @@ __device__ __forceinline__ void boundary_state_rot(const LawP& L, int d, const i
   }
 }
 
-// The other numerical fluxes of a face node, on rotated states (direction 0)
-template <int LAW, int DIM>
-__device__ __forceinline__ void line_flux_dir(const LawP& L, int kind, bool f32, double sgn, const double* qm,
-                                              const double* am, const double* qp, const double* ap, double* nf) {
-  if (!f32 || !surface_flux32<LAW, DIM>(L, kind, 0, sgn, qm, am, qp, ap, nf))
-    surface_flux<LAW, DIM>(L, kind, 0, sgn, qm, am, qp, ap, nf);
-}
-// every flux, chosen at run time: one out-of-line copy for each precision form (one
-// for both cost the FP64 operators 1 to 5 %)
+// The other numerical fluxes of a face node.  FP32-flux forms of Euler and
+// Euler-gravity: components in x, y, z order with the direction a constant, so
+// their FP32 sums round as in the node-per-thread kernels; else rotated
+// (direction 0).
 template <int LAW, int DIM, bool F32>
-__device__ __noinline__ void line_flux_any(const LawP& L, int kind, double sgn, const double* qm, const double* am,
-                                           const double* qp, const double* ap, double* nf) {
-  line_flux_dir<LAW, DIM>(L, kind, F32, sgn, qm, am, qp, ap, nf);
+__device__ __forceinline__ void line_flux_dir(const LawP& L, int kind, int d, double sgn, const double* qm,
+                                              const double* am, const double* qp, const double* ap, double* nf) {
+  auto one = [&](auto dc) {
+    constexpr int D_ = decltype(dc)::value;
+    if (!F32 || !surface_flux32<LAW, DIM>(L, kind, D_, sgn, qm, am, qp, ap, nf))
+      surface_flux<LAW, DIM>(L, kind, D_, sgn, qm, am, qp, ap, nf);
+  };
+  if constexpr (F32 && LAW != LAW_SW) {
+    if (DIM > 2 && d == 2)
+      one(std::integral_constant<int, (DIM > 2 ? 2 : 0)>{});
+    else if (DIM > 1 && d == 1)
+      one(std::integral_constant<int, (DIM > 1 ? 1 : 0)>{});
+    else
+      one(std::integral_constant<int, 0>{});
+  } else {
+    one(std::integral_constant<int, 0>{});
+  }
+}
+// every flux, chosen at run time: one out-of-line copy
+template <int LAW, int DIM, bool F32>
+__device__ __noinline__ void line_flux_any(const LawP& L, int kind, int d, double sgn, const double* qm,
+                                           const double* am, const double* qp, const double* ap, double* nf) {
+  line_flux_dir<LAW, DIM, F32>(L, kind, d, sgn, qm, am, qp, ap, nf);
+}
+template <int LAW, int DIM, bool F32, int SF>
+__device__ __forceinline__ void line_flux(const LawP& L, int kind, int d, double sgn, const double* qm,
+                                          const double* am, const double* qp, const double* ap, double* nf) {
+  if constexpr (SF >= 0)
+    line_flux_dir<LAW, DIM, F32>(L, SF, d, sgn, qm, am, qp, ap, nf);
+  else
+    line_flux_any<LAW, DIM, F32>(L, kind, d, sgn, qm, am, qp, ap, nf);
 }
 
 // rotated component c of direction d: the normal component first
@@ -467,6 +520,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
   constexpr int NFP = ipow(NQ, DIM - 1);
   constexpr int NXA = S::NXA;
   constexpr int DZ = DIM - 1;
+  constexpr bool F32S = S::F32 && !S::SW;  // FP32 face sums: components in x, y, z order
   const int epi = A.epi;
   const int sflux = SF >= 0 ? SF : A.sflux;
   const int lin_sflux = SF >= 0 ? SF : A.lin_sflux;
@@ -509,8 +563,9 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     int rot[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) rot[c] = line_rot<DIM>(c, d);
-    // its two faces: neighbours, then their traces (rotated).  A boundary face
-    // loads its own trace, so the loads are free of branches.
+    // its two faces: neighbours, then their traces (rotated; x, y, z order in
+    // the FP32-flux forms).  A boundary face loads its own trace, so the loads
+    // are free of branches.
     int nv[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) nv[i] = __ldg(A.nbr + 6 * e + 2 * d + i);
@@ -524,7 +579,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
                (hi ? NQ - 1 : 0) * line_stride<NQ, DIM>(d, NQ);
       qp[i][0] = __ldg(A.q[0] + nid[i]);
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) qp[i][1 + c] = __ldg(A.q[1 + rot[c]] + nid[i]);
+      for (int c = 0; c < DIM; ++c) qp[i][1 + c] = __ldg(A.q[1 + (F32S ? c : rot[c])] + nid[i]);
       qp[i][DIM + 1] = __ldg(A.q[DIM + 1] + nid[i]);
       ap[i] = 0.0;
       if (LAW == LAW_EG || (S::SW && L.swtopo)) ap[i] = __ldg(A.aux + nid[i]);
@@ -579,7 +634,24 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
             double t = fma(-0.5, dot<DIM>(q[r] + 1, u), q[r][DIM + 1]);
             if constexpr (S::EG) t = fma(-q[r][0], a0, t);
             const double p = __dmul_rn(L.gamma - 1.0, t);
-            if constexpr (VK == VK_WEAK) {
+            if constexpr (S::F32) {
+              sx[0] = p;
+              if constexpr (VK == VK_EC32) {
+                const double pr = __dmul_rn(p, rinv);
+                sx[NPL] = 0.5 * rcp_cheb(pr);
+                sx[2 * NPL] = pr;
+              }
+              if constexpr (S::EG) sx[(S::ND - 1) * NPL] = a0;
+              const float rinvf = (float)rinv;
+              float uu = 0.f;
+#pragma unroll
+              for (int c = 0; c < DIM; ++c) {
+                const float uf = (float)q[r][1 + c] * rinvf;
+                sf[c * NPL] = uf;
+                uu += uf * uf;
+              }
+              sf[DIM * NPL] = (VK == VK_EC32) ? uu : (float)q[r][DIM + 1] * rinvf;
+            } else if constexpr (VK == VK_WEAK) {
               sx[0] = rinv;
               sx[NPL] = L.pde ? p - __ldg(A.aux + (DIM + 2) * A.stride + g0 + v) : p;
               sx[2 * NPL] = q[r][DIM + 1] + p;
@@ -614,6 +686,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     double* const sq = s0 + es * slotsz;
     double* const sx = sq + OX;
     const int base = line_base<NQ, DIM>(d, l, ROW), sd = line_stride<NQ, DIM>(d, ROW);
+    constexpr bool XYZ = VK == VK_EC32 && !S::SW;  // accumulators in x, y, z order
     double T[NQ][NS], X[NQ];
 #pragma unroll
     for (int a = 0; a < NQ; ++a) {
@@ -627,17 +700,22 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         const int nm = base + (i ? (NQ - 1) * sd : 0);
         qm[0] = sq[nm];
 #pragma unroll
-        for (int c = 0; c < DIM; ++c) qm[1 + c] = sq[(1 + rot[c]) * NPL + nm];
+        for (int c = 0; c < DIM; ++c) qm[1 + c] = sq[(1 + (F32S ? c : rot[c])) * NPL + nm];
         qm[DIM + 1] = sq[(DIM + 1) * NPL + nm];
 #pragma unroll
         for (int k = 0; k < NAM; ++k) am[k] = 0.0;
         if (LAW == LAW_EG || S::SW) {
           am[0] = sx[(S::ND - 1) * NPL + nm];
-          if (LAW == LAW_EG) am[0] = 4.0 * am[0];
+          if (LAW == LAW_EG && !S::F32) am[0] = 4.0 * am[0];
         }
       };
       auto bc = [&](int i, const LawP& Lb, const double* qm, double* qb) {
-        boundary_state_rot<LAW, DIM>(Lb, d, rot, 0, i ? 1.0 : -1.0, nv[i] - NBR_BOUNDARY, qm, qb);
+        if constexpr (F32S) {
+          const int id[3] = {0, 1, 2};
+          boundary_state_rot<LAW, DIM>(Lb, d, id, d, i ? 1.0 : -1.0, nv[i] - NBR_BOUNDARY, qm, qb);
+        } else {
+          boundary_state_rot<LAW, DIM>(Lb, d, rot, 0, i ? 1.0 : -1.0, nv[i] - NBR_BOUNDARY, qm, qb);
+        }
       };
       // pde_level_balance: the reference state too
       auto aux = [&](int i, double* am, double* apv) {
@@ -668,18 +746,24 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         const double sgn = i ? 1.0 : -1.0;
         if constexpr (RUS)
           line_rusanov<LAW, DIM>(L, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
-        else if constexpr (SF >= 0)
-          line_flux_dir<LAW, DIM>(L, SF, S::F32, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
-        else if (S::F32 || (!S::SW && A.sf32))
-          line_flux_any<LAW, DIM, true>(L, sflux, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
         else
-          line_flux_any<LAW, DIM, false>(L, sflux, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
+          line_flux<LAW, DIM, S::F32, SF>(L, sflux, d, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         double(&Te)[NS] = T[i ? NQ - 1 : 0];
 #pragma unroll
         for (int s = 0; s < NS; ++s) Te[s] = __dmul_rn(-lift_end, nf[i][s]);
+        if constexpr (F32S && !XYZ) {  // fluxes in x, y, z order, accumulators rotated
+#pragma unroll
+          for (int c = 0; c < DIM; ++c) {
+            double f = nf[i][1];
+#pragma unroll
+            for (int k = 1; k < DIM; ++k)
+              if (rot[c] == k) f = nf[i][1 + k];
+            Te[1 + c] = __dmul_rn(-lift_end, f);
+          }
+        }
       }
     }
     if constexpr (FUSE) {
@@ -708,8 +792,14 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           for (int c = 0; c < DIM; ++c) qo[1 + c] = sq[(1 + rot[c]) * NPL + nm];
           qo[DIM + 1] = sq[(DIM + 1) * NPL + nm];
           if (inner) {
+            // (the traces above are in x, y, z order in the FP32-flux forms)
 #pragma unroll
             for (int s = 0; s < NS; ++s) qn[s] = qp[i][s];
+            if constexpr (F32S) {
+              qn[1] = qp[i][1 + DZ];
+#pragma unroll
+              for (int c = 1; c < DIM; ++c) qn[1 + c] = qp[i][c];
+            }
           } else {
             boundary_state_rot<LAW_LEG, DIM>(A.lin_law, d, rot, 0, sgn, nv[i] - NBR_BOUNDARY, qo, qn);
           }
@@ -770,12 +860,12 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     // B lie, from the high words (monotonic for positive values; NaN and
     // non-positive values fail both tests)
     int form = 0;
-    if constexpr (VK == VK_EC && !S::SW) {
+    if constexpr ((VK == VK_EC || VK == VK_EC32) && !S::SW) {
       int rlo = 0x7fffffff, rhi = -0x7fffffff - 1, blo = rlo, bhi = rhi;
 #pragma unroll
       for (int a = 0; a < NQ; ++a) {
         const int n = base + a * sd;
-        const int hr = __double2hiint(sq[n]), hb = __double2hiint(sx[DIM * NPL + n]);
+        const int hr = __double2hiint(sq[n]), hb = __double2hiint(sx[(VK == VK_EC ? DIM : 1) * NPL + n]);
         rlo = min(rlo, hr);
         rhi = max(rhi, hr);
         blo = min(blo, hb);
@@ -784,7 +874,10 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
       const double rmax = __hiloint2double(rhi + 1, 0), bmax = __hiloint2double(bhi + 1, 0);
       const double rmin = __hiloint2double(rlo, 0), bmin = __hiloint2double(blo, 0);
       const bool near = rmax < 1.2 * rmin && bmax < 1.2 * bmin;
-      form = near ? 0 : rmax < 3.0 * rmin && bmax < 3.0 * bmin ? 1 : 2;
+      if constexpr (VK == VK_EC32)
+        form = DIM == 3 && __all_sync(0xffffffffu, near) ? 0 : 2;  // (every lane of the CTA is here)
+      else
+        form = near ? 0 : rmax < 3.0 * rmin && bmax < 3.0 * bmin ? 1 : 2;
     }
     if (act) {
       // ---- two-point fluxes of the line's pairs, or the weak form's rows
@@ -798,20 +891,34 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           line_pairs<LAW, DIM, VK, NQ, 1>(A, c0, sq, sx, base, sd, rot, d, T, X);
         else
           line_pairs<LAW, DIM, VK, NQ, 2>(A, c0, sq, sx, base, sd, rot, d, T, X);
+      } else if constexpr (VK == VK_EC32 && !S::SW) {
+        const double c0 = 1.0 / (L.gamma - 1.0);
+        if (DIM == 3 && form == 0)
+          line_pairs<LAW, DIM, VK, NQ, (DIM == 3 ? 0 : 2)>(A, c0, sq, sx, base, sd, rot, d, T, X);
+        else
+          line_pairs<LAW, DIM, VK, NQ, 2>(A, c0, sq, sx, base, sd, rot, d, T, X);
       } else {
         const double c0 = S::SW ? 0.5 * L.grav : 1.0 / (L.gamma - 1.0);
         line_pairs<LAW, DIM, VK, NQ, 0>(A, c0, sq, sx, base, sd, rot, d, T, X);
       }
 #pragma unroll
       for (int a = 0; a < NQ; ++a) {
-        if constexpr (S::XTRA && VK != VK_KG) {
+        if constexpr (S::XTRA && VK != VK_KG && VK != VK_KG32) {
           const int n = base + a * sd;
           double t = X[a];
           if constexpr (S::SW)
             t = L.swtopo ? __dmul_rn(t, 0.5 * L.grav * sq[n]) : 0.0;
           else if constexpr (VK == VK_EC)
             t = __dmul_rn(t, sx[(DIM + 1) * NPL + n]);
-          T[a][1] -= t;
+          else if constexpr (VK == VK_EC32)
+            t = __dmul_rn(t, sx[2 * NPL + n]);
+          if constexpr (XYZ) {
+#pragma unroll
+            for (int c = 0; c < DIM; ++c)
+              if (c == d) T[a][1 + c] -= t;
+          } else {
+            T[a][1] -= t;
+          }
         }
 #pragma unroll
         for (int s = 0; s < NS; ++s) T[a][s] = __dmul_rn(T[a][s], gd);
@@ -825,7 +932,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         for (int a = 0; a < NQ; ++a)
 #pragma unroll
           for (int s = 0; s < NS; ++s) {
-            const int c = (s == 0 || s == DIM + 1) ? s : 1 + rot[s - 1];
+            const int c = (s == 0 || s == DIM + 1 || XYZ) ? s : 1 + rot[s - 1];
             B[c * NPL + base + a * sd] = T[a][s];
           }
       }
@@ -838,7 +945,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           for (int a = 0; a < NQ; ++a)
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-              const int c = (s == 0 || s == DIM + 1) ? s : 1 + (s - 1 + dd) % DIM;
+              const int c = (s == 0 || s == DIM + 1 || XYZ) ? s : 1 + (s - 1 + dd) % DIM;
               double* const o = sx + c * NPL + base + a * sd;
               *o = dd == 0 ? T[a][s] : *o + T[a][s];
             }
@@ -1017,8 +1124,6 @@ template <int LAW, int DIM, int VK, bool FUSE, int SF, bool PERSIST> tend_launch
   return nullptr;
 }
 
-// the volume kind that a line kernel runs for the one asked for
-int fd_volume_kind(int law, int vk);
 tend_launch_fn pick_fd(int law, int dim, int vk, int nq, int sflux);
 tend_launch_fn pick_fd_fused(int dim, int vk, int nq, int sflux, int lin_sflux);
 tend_launch_fn pick_fd_persistent(int law, int dim, int vk, int nq, int sflux, bool fused, int lin_sflux);

@@ -1,6 +1,7 @@
 // fd_kernel instantiations (parallel compilation):
 //   2-D Euler-gravity, EC volume flux, Rusanov surface flux
 //   2-D Euler-gravity, EC volume flux, every surface flux
+//   2-D Euler-gravity, FP32-flux EC volume flux, every surface flux
 #include "atb_fd.cuh"
 
 namespace atb {
@@ -9,5 +10,8 @@ tend_launch_fn fd_eg2_ec_rus(int nq) {
 }
 tend_launch_fn fd_eg2_ec_any(int nq) {
   return fd_pick<LAW_EG, 2, VK_EC, false, -1, false>(nq);
+}
+tend_launch_fn fd_eg2_ec32_any(int nq) {
+  return fd_pick<LAW_EG, 2, VK_EC32, false, -1, false>(nq);
 }
 }  // namespace atb

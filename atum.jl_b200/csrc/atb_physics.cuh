@@ -516,7 +516,9 @@ template <class T> __device__ __forceinline__ T series_G(T u) {
 // series correction, so the hydrostatic balance between the pressure and
 // gravity terms is carried in FP64 while every division, logarithm and
 // advective product is FP32.  Returns FP64 row values and b_avg * rho_log.
-template <int LAW, int DIM>
+// NEAR: the caller knows that both logarithmic means of every pair it
+// evaluates are on their series branch (the same values, no branch per pair).
+template <int LAW, int DIM, bool NEAR = false>
 __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1, double b1, const float* u1,
                                          float uu1, double Phi1, double r2, double p2, double b2,
                                          const float* u2, float uu2, double Phi2, double* f, double* xtra) {
@@ -527,7 +529,7 @@ __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1
   const float ur = fr * fr, ub = fb * fb;
   double rho_log;
   float cterm;
-  if (ur < 1e-2f && ub < 1e-2f) {
+  if (NEAR || (ur < 1e-2f && ub < 1e-2f)) {
     // 1 - G(u) = u/3 + 4u^2/45 + 44u^3/945 + ... (the terms of series_G)
     const float cr = ur * (1.f / 3.f + ur * (4.f / 45.f + ur * (44.f / 945.f + ur * (428.f / 14175.f +
                      ur * (10196.f / 467775.f + ur * (10719068.f / 638512875.f + ur * (25865068.f / 1915538625.f)))))));

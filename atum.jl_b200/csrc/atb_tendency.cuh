@@ -67,7 +67,6 @@ struct TendArgs {
   double cfd[64];      // Cfd again for the flux-differencing kernels (Nq <= 8): constant-bank operands
   LawP law;
   int dirs, sflux, epi;
-  int sf32;            // line kernels: the numerical flux in its FP32-flux form (those chosen at run time)
   double a, bdt;
   const double* dte;  // per-element time step (batched instances), or null
   // EPI_ARK accumulators (acc[j][0] null: inactive; accin[j][0] null: base Q)

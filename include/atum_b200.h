@@ -62,7 +62,6 @@ extern "C" {
 #define ATB_SRC_CORIOLIS 1
 /* precision forms */
 #define ATB_PREC_FP64 0
-/* permits FP32 flux arithmetic; terms that are faster in FP64 stay FP64 */
 #define ATB_PREC_FP32FLUX 1
 /* solvers: src/odesolvers.jl */
 #define ATB_LSRK54 0
