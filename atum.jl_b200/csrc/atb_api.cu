@@ -148,6 +148,7 @@ struct atb_op {
   std::vector<int> col_e0;    // bottom element of every vertical column
   bool cols_uniform = true;   // every instance has the same element counts
   int npre = 0, npv = 0;
+  int small = 0;     // threads of their mode for grids of one wave (fd_small), 0: not used
   bool fd = false;   // flux differencing by the flux-differencing kernels (atb_fd.cuh)
   // page-locked geometry staging of pools: a ring of kGeoRing areas, each
   // reused once the copies out of it have run, so a placement waits only for
@@ -234,6 +235,7 @@ void fill_args(const atb_op* op, TendArgs& A) {
   A.law = op->law;
   A.dirs = op->dirs;
   A.sflux = op->sflux;
+  A.small = op->small;
   A.stride = op->stride();
   A.a = 0;
   A.bdt = 0;
@@ -633,6 +635,7 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
     // Cfd, or Cw for the weak form
     std::copy_n(tab.begin() + (vk == VK_WEAK ? Nq * Nq : 0), Nq * Nq, op->cfd);
     op->E = fd_default_elements(Nq, dim, fd_limit(op), K, nsm, false);
+    op->small = fd_small(d->law, dim, vk, Nq, sf, K, nsm);
   }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
@@ -749,6 +752,7 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
     }
   op->curved = true;
   op->fd = fd;  // its kernels and their shapes are the curved ones
+  op->small = 0;
   if (fd) std::memcpy(op->cfd, op->D.data(), (size_t)Nq * Nq * sizeof(double));  // D[i][m]
   op->launch = fn;
   // aux the kernels read: Phi (fluxes, wave speeds), grad Phi (weak-form
@@ -921,30 +925,41 @@ extern "C" int atb_op_autotune(atb_op* op, const double* const* q, double* scrat
   cudaStream_t st = (cudaStream_t)stream;
   double* out[5];
   for (int s = 0; s < 5; ++s) out[s] = scratch + (size_t)(s < op->ns ? s : 0) * op->stride();
-  const int E0 = op->E;
-  int best = E0;
+  // the mode for grids of one wave, where the operator takes it, is a candidate too
+  const int E0 = op->E, small0 = op->small;
+  int best = E0, best_small = small0;
   float best_ms = 1e30f;
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
-  for (int E = 1; op->fd ? E <= fd_limit(op) : (cta_threads(E, op->Np) <= 512 && E <= 16); ++E) {
-    if (op_smem(op, E) > 200 * 1024) break;
-    op->E = E;
-    op->smem = op_smem(op, E);
+  for (int E = small0 ? 0 : 1; op->fd ? E <= fd_limit(op) : (cta_threads(E, op->Np) <= 512 && E <= 16); ++E) {
+    const int Ec = E ? E : E0;
+    if (op_smem(op, Ec) > 200 * 1024) break;
+    op->E = Ec;
+    op->smem = op_smem(op, Ec);
+    op->small = E ? 0 : small0;
     int rc = run_tendency(op, EPI_SET, q, out, nullptr, 0, 0, st);  // warm-up
-    if (rc) { op->E = E0; op->smem = op_smem(op, E0); cudaEventDestroy(a); cudaEventDestroy(b); return rc; }
+    if (rc) {
+      op->E = E0;
+      op->smem = op_smem(op, E0);
+      op->small = small0;
+      cudaEventDestroy(a);
+      cudaEventDestroy(b);
+      return rc;
+    }
     CK(cudaEventRecord(a, st));
     for (int r = 0; r < 5; ++r) run_tendency(op, EPI_SET, q, out, nullptr, 0, 0, st);
     CK(cudaEventRecord(b, st));
     CK(cudaEventSynchronize(b));
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
-    if (ms < best_ms) { best_ms = ms; best = E; }
+    if (ms < best_ms) { best_ms = ms; best = Ec; best_small = op->small; }
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   op->E = best;
   op->smem = op_smem(op, best);
+  op->small = best_small;
   if (chosen) *chosen = best;
   return check_launch("autotune");
 }
@@ -969,6 +984,7 @@ extern "C" int atb_op_set_launch(atb_op* op, int elements_per_cta) {
     return fail(ATB_ERR_INVALID, "bad elements per CTA");
   op->E = elements_per_cta;
   op->smem = op_smem(op, elements_per_cta);
+  op->small = 0;
   return ATB_OK;
 }
 

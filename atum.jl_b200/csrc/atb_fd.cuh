@@ -153,6 +153,72 @@ inline size_t fd_smem_bytes(int law, int dim, int vk, int nq, int E, bool fuse) 
   return sizeof(double) * ((size_t)nq * nq + 2 + (size_t)E * slot);
 }
 
+// ---------------------------------------------------- grids of one wave
+// A line's thread evaluates its pairs one after the other, 28 at Nq = 8, and both
+// face fluxes: where the whole grid is resident at once, a launch takes as long as
+// that chain.  The SMALL mode of the kernel has one element per CTA and spreads
+// the pairs and the faces of its lines over all threads, values through shared
+// memory; the node's thread sums them in the order of the line's thread.  The same
+// operations on the same values give the same bits, so the mode may be chosen by
+// the element count.  us per LSRK54 stage, line per thread / SMALL:
+//   2-D Euler-gravity FP64 N = 7, 8x8 elements 7.9 / 4.9, 24x24 8.8 / 7.1 (96
+//   threads; 10.2 with 448), 40x40 11.6 / 16.7; FP32 flux 8x8 11.6 / 5.6, 32x32
+//   15.1 / 11.9; Roe flux 8x8 11.5 / 6.8; 2-D Euler FP64 N = 5, 8x8 5.1 / 4.3,
+//   N = 4 3.7 / 4.3.  3-D: FP64 pairs gain nothing (N = 4, 27 elements 4.9 / 5.6);
+//   FP32-flux EC, ARK23 step, 3^3 N = 4 51 / 33, N = 6 95 / 56, 6^3 N = 7 112 /
+//   149; weak form with Roe's flux, 5^3 N = 4 9.3 / 6.9.
+__host__ __device__ constexpr int small_pairs(int nq) { return nq * (nq - 1) / 2; }
+// directions whose pairs share the buffer: all, while they leave room for two CTAs
+__host__ __device__ constexpr int small_batch(int nq, int dim) { return dim == 2 || nq <= 6 ? dim : 1; }
+// a thread for every node and face, the most for the pairs
+__host__ __device__ constexpr int small_least(int nq, int dim) {
+  const int faces = 2 * line_count(nq, dim), nodes = ipow(nq, dim);
+  return ((faces > nodes ? faces : nodes) + 31) / 32 * 32;
+}
+__host__ __device__ constexpr int small_threads(int nq, int dim) {
+  const int pairs = (line_count(nq, dim) * small_pairs(nq) + 31) / 32 * 32;
+  const int cap = dim == 2 ? 448 : nq <= 5 ? 288 : nq == 6 ? 384 : 512;
+  const int most = pairs < cap ? pairs : cap;
+  return most > small_least(nq, dim) ? most : small_least(nq, dim);
+}
+// where it is compiled (sf < 0: the surface flux chosen at run time)
+__host__ __device__ constexpr bool fd_has_small(int law, int dim, int vk, int sf) {
+  if (dim == 2) return law == LAW_EULER || law == LAW_EG;
+  return law == LAW_EG && (vk == VK_EC32 || (vk == VK_WEAK && sf < 0));
+}
+// Threads per CTA of the SMALL mode, 0 where a thread per line is faster (measured
+// per order; K elements, nsm multiprocessors): 2-D up to four elements per
+// multiprocessor, where FP64 pairs with Rusanov's flux are many (Nq >= 6) or the
+// chain is long otherwise (Nq >= 4), and seven for the longest; 3-D one, or as far
+// as its CTAs are resident together.  Fewer threads as the elements get more.
+inline int fd_small(int law, int dim, int vk, int nq, int sf, int K, int nsm) {
+  const bool any = sf != F_RUSANOV;
+  if (!fd_has_small(law, dim, vk, any ? -1 : sf)) return 0;
+  const bool slow = vk == VK_EC32 || any;
+  int most = 0;  // elements per two multiprocessors
+  if (dim == 2)
+    most = nq == 8 && slow ? 14 : nq >= 6 || (slow && nq >= 4) ? 8 : 0;
+  else if (vk == VK_WEAK)
+    most = nq == 4 ? 8 : nq == 5 || nq == 6 ? 3 : nq == 7 ? 2 : 0;
+  else
+    most = nq == 5 ? 3 : nq >= 4 && nq <= 7 ? 2 : 0;
+  if (2LL * K > (long long)most * nsm) return 0;
+  const int cap = K <= nsm ? small_threads(nq, dim) : K <= 4 * nsm ? 96 : 64;
+  const int least = small_least(nq, dim), full = small_threads(nq, dim);
+  const int t = cap < full ? cap : full;
+  return t > least ? t : least;
+}
+// doubles of shared memory: tables, the element, face fluxes, line forms and pair
+// numbers, pair values (NS and the extra one)
+__host__ __device__ constexpr int small_slot(int ns, int nxa, int nq, int dim, bool fuse) {
+  return (ns + nxa + (fuse ? 2 + ns : 0)) * line_nodes(nq, dim);
+}
+__host__ __device__ constexpr int small_doubles(int ns, int nxa, int nq, int dim, bool fuse, bool pairs) {
+  const int nl = line_count(nq, dim), np = small_pairs(nq);
+  return 2 * nq * nq + 2 + small_slot(ns, nxa, nq, dim, fuse) + 2 * nl * ns + (nl + np + 1) / 2 +
+         (pairs ? small_batch(nq, dim) * ipow(nq, dim - 1) * np * (ns + 1) : 0);
+}
+
 // ------------------------------------------------------------ pair fluxes
 // Point values of one node as a pair flux reads them; velocities rotated
 // (normal component first) in the FP64 forms.
@@ -208,6 +274,54 @@ __device__ __forceinline__ void line_load(LinePt<LAW, DIM, VK>& P, const double*
   }
 }
 
+// The FP32-flux EC pair of ec_vol32 for a line whose values lie within a factor 1.2
+// (both logarithmic means on their series branch): the same FP32 operations and
+// roundings without a branch, a call or a division, so that a line's pairs overlap;
+// the quotients of one divisor share its reciprocal.  (2-D Euler N = 7, 24x24
+// elements: 18.3 -> 11.1 us per LSRK54 stage; 3-D Euler-gravity N = 5, 10^3: 30.7 ->
+// 25.3.  What is left is conversions, 14 or 15 a pair.)
+template <int LAW, int DIM>
+__device__ __forceinline__ void ec_line32(float igm1, int d, const LinePt<LAW, DIM, VK_EC32>& P,
+                                          const LinePt<LAW, DIM, VK_EC32>& Q, double* f, double* xtra) {
+  const double rs64 = P.r + Q.r, bs64 = P.b + Q.b;
+  const double rho_avg = rs64 * 0.5, p_avg = (P.p + Q.p) * 0.5;
+  const float rs = (float)rs64, rd = (float)(P.r - Q.r), bs = (float)bs64, bd = (float)(P.b - Q.b);
+  const float ir = rcp32(rs), ib = rcp32(bs);
+  const float fr = div32(rd, rs, ir), fb = div32(bd, bs, ib);
+  const float ur = fr * fr, ub = fb * fb;
+  const float cr = ur * (1.f / 3.f + ur * (4.f / 45.f + ur * (44.f / 945.f + ur * (428.f / 14175.f +
+                   ur * (10196.f / 467775.f + ur * (10719068.f / 638512875.f + ur * (25865068.f / 1915538625.f)))))));
+  const double rho_log = rho_avg - rho_avg * (double)cr;
+  const float cterm = div32(series_F(ub) * igm1, bs, ib);
+  const double corr = (double)div32((float)(P.p - Q.p) * -bd, 2.f * bs, 0.5f * ib);
+  const double pc = p_avg - corr;
+  float ua[DIM];
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) ua[c] = 0.5f * (P.uf[c] + Q.uf[c]);
+  const float rl = (float)rho_log;
+  float ud = ua[0];
+#pragma unroll
+  for (int c = 1; c < DIM; ++c)
+    if (c == d) ud = ua[c];
+  const float frd = ud * rl;
+  f[0] = (double)frd;
+  float mu = 0.f;
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    const float m = ud * (ua[c] * rl);
+    f[1 + c] = (double)m;
+    mu += m * ua[c];
+  }
+#pragma unroll
+  for (int c = 0; c < DIM; ++c)
+    if (c == d) f[1 + c] += pc;
+  mu += (float)pc * ud;
+  float c1 = cterm - 0.25f * (P.xf + Q.xf);
+  if (LAW == LAW_EG) c1 += (float)((P.ph + Q.ph) * 0.5);
+  f[DIM + 1] = (double)(c1 * frd + mu);
+  *xtra = (bs64 * 0.5) * rho_log;
+}
+
 // Symmetric two-point flux f (components rotated: normal momentum at 1, except
 // VK_EC32, x y z order) and the extra value x, antisymmetric in the pair.
 //   EC: rho_log, p_c = rho_avg / (2 b_avg), and the energy flux in the form
@@ -218,11 +332,8 @@ __device__ __forceinline__ void line_load(LinePt<LAW, DIM, VK>& P, const double*
 //   TIER: the line's values lie within a factor 1.2 (0), within a factor 3 (1: a
 //   longer polynomial; the core of a vortex on a coarse grid), or further apart
 //   (2: logarithms).  The form depends on the line alone, so results do not
-//   depend on the launch shape.  The FP32-flux form's two versions (0: every
-//   pair on the series branch; 2: a branch per pair) give the same values, so
-//   there a warp takes one for all its lines; in 2-D only the second is
-//   compiled (the first gains nothing on a large grid and the second copy of
-//   the unrolled pairs costs a small one a third of its step).
+//   depend on the launch shape.  FP32-flux form: 0 (ec_line32), or a branch per
+//   pair (2).
 template <int LAW, int DIM, int VK, int TIER>
 __device__ __forceinline__ void line_pair(const LawP& L, double c0, int d, const LinePt<LAW, DIM, VK>& P,
                                           const LinePt<LAW, DIM, VK>& Q, double* f, double& x) {
@@ -251,8 +362,11 @@ __device__ __forceinline__ void line_pair(const LawP& L, double c0, int d, const
     // ec_vol32 with the direction given at run time (the FP32 sums stay in
     // x, y, z order)
     double xr;
-    ec_vol32<LAW, DIM, TIER == 0>((float)c0, d, P.r, P.p, P.b, P.uf, P.xf, S::EG ? P.ph : 0.0, Q.r, Q.p, Q.b, Q.uf, Q.xf,
-                       S::EG ? Q.ph : 0.0, f, &xr);
+    if constexpr (TIER == 0)
+      ec_line32<LAW, DIM>((float)c0, d, P, Q, f, &xr);
+    else
+      ec_vol32<LAW, DIM>((float)c0, d, P.r, P.p, P.b, P.uf, P.xf, S::EG ? P.ph : 0.0, Q.r, Q.p, Q.b, Q.uf, Q.xf,
+                         S::EG ? Q.ph : 0.0, f, &xr);
     if constexpr (S::EG) x = xr * (P.ph - Q.ph);
   } else if constexpr (VK == VK_KG) {
     const double ravg = 0.5 * (P.r + Q.r);
@@ -301,6 +415,38 @@ __device__ __forceinline__ void line_pair(const LawP& L, double c0, int d, const
   }
 }
 
+// The form (TIER) of a line's logarithmic means: how far apart its densities and B lie,
+// from the high words (monotonic for positive values).  The polynomial forms are
+// for positive numbers of ordinary size: their common reciprocal of (R B)^2 stays a
+// normal number (FP32: so do the quotients).
+template <int LAW, int DIM, int VK, int NQ>
+__device__ __forceinline__ int line_form(const double* sq, const double* sx, int base, int sd) {
+  int form = 0;
+  if constexpr ((VK == VK_EC || VK == VK_EC32) && LAW != LAW_SW) {
+    constexpr int npl = line_nodes(NQ, DIM);
+    int rlo = 0x7fffffff, rhi = -0x7fffffff - 1, blo = rlo, bhi = rhi;
+#pragma unroll
+    for (int a = 0; a < NQ; ++a) {
+      const int n = base + a * sd;
+      const int hr = __double2hiint(sq[n]), hb = __double2hiint(sx[(VK == VK_EC ? DIM : 1) * npl + n]);
+      rlo = min(rlo, hr);
+      rhi = max(rhi, hr);
+      blo = min(blo, hb);
+      bhi = max(bhi, hb);
+    }
+    const double rmax = __hiloint2double(rhi + 1, 0), bmax = __hiloint2double(bhi + 1, 0);
+    const double rmin = __hiloint2double(rlo, 0), bmin = __hiloint2double(blo, 0);
+    constexpr int EX = VK == VK_EC32 ? 100 : 240;  // between 2^-EX and 2^EX
+    const bool plain = min(rlo, blo) >= ((1023 - EX) << 20) && max(rhi, bhi) < ((1023 + EX) << 20);
+    const bool near = plain && rmax < 1.2 * rmin && bmax < 1.2 * bmin;
+    if constexpr (VK == VK_EC32)
+      form = near ? 0 : 2;
+    else
+      form = near ? 0 : plain && rmax < 3.0 * rmin && bmax < 3.0 * bmin ? 1 : 2;
+  }
+  return form;
+}
+
 // every pair of the line, both nodes' rows of Cfd (in the parameters: constant-
 // bank operands)
 template <int LAW, int DIM, int VK, int NQ, int TIER>
@@ -346,20 +492,23 @@ __device__ __forceinline__ void line_pairs(const TendArgs& A, double c0, const d
 
 // Weak form: D^T-weighted flux rows of the line's nodes (Cw in the parameters),
 // [m_n, m u_n + p n, (rho e + p) u_n] rotated
+template <int DIM>
+__device__ __forceinline__ void weak_row(const double* sq, const double* sx, int npl, int n, const int* rot, double* f) {
+  f[0] = sq[(1 + rot[0]) * npl + n];
+  const double un = __dmul_rn(f[0], sx[n]);
+  f[1] = fma(f[0], un, sx[npl + n]);
+#pragma unroll
+  for (int c = 1; c < DIM; ++c) f[1 + c] = __dmul_rn(sq[(1 + rot[c]) * npl + n], un);
+  f[DIM + 1] = __dmul_rn(sx[2 * npl + n], un);
+}
 template <int DIM, int NQ>
 __device__ __forceinline__ void line_weak(const TendArgs& A, const double* sq, const double* sx, int base, int sd,
                                           const int* rot, double (*T)[DIM + 2]) {
   constexpr int npl = line_nodes(NQ, DIM);
 #pragma unroll
   for (int m = 0; m < NQ; ++m) {
-    const int n = base + m * sd;
     double f[DIM + 2];
-    f[0] = sq[(1 + rot[0]) * npl + n];
-    const double un = __dmul_rn(f[0], sx[n]);
-    f[1] = fma(f[0], un, sx[npl + n]);
-#pragma unroll
-    for (int c = 1; c < DIM; ++c) f[1 + c] = __dmul_rn(sq[(1 + rot[c]) * npl + n], un);
-    f[DIM + 1] = __dmul_rn(sx[2 * npl + n], un);
+    weak_row<DIM>(sq, sx, npl, base + m * sd, rot, f);
 #pragma unroll
     for (int a = 0; a < NQ; ++a)
 #pragma unroll
@@ -508,9 +657,11 @@ __device__ __forceinline__ int line_stride(int d, int row) {
   return d == 0 ? 1 : d == 1 ? row : row * NQ;
 }
 
-template <int LAW, int DIM, int VK, int NQ, bool FUSE, int SF, bool PERSIST>
-__global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(LAW, DIM, VK, NQ).min_blocks)
+template <int LAW, int DIM, int VK, int NQ, bool FUSE, int SF, bool PERSIST, bool SMALL = false>
+__global__ void __launch_bounds__(SMALL ? small_threads(NQ, DIM) : fd_cfg(LAW, DIM, VK, NQ).max_threads,
+                                  SMALL ? 1 : fd_cfg(LAW, DIM, VK, NQ).min_blocks)
     fd_kernel(const __grid_constant__ TendArgs A) {
+  static_assert(!(SMALL && PERSIST), "one launch mode");
   using S = LineShape<LAW, DIM, VK>;
   constexpr int NS = S::NS;
   constexpr int NAM = NAuxMax<LAW, DIM>::v;
@@ -524,15 +675,29 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
   const int epi = A.epi;
   const int sflux = SF >= 0 ? SF : A.sflux;
   const int lin_sflux = SF >= 0 ? SF : A.lin_sflux;
-  const int E = A.E;
+  const int E = SMALL ? 1 : A.E;
   extern __shared__ double sm[];
   double* const sW = sm;  // Cw (the fused linear operator), lift
   constexpr int NB = fd_cfg(LAW, DIM, VK, NQ).bufs;
   static_assert(NB == 1 || NB == DIM, "one accumulator array, or one per direction");
-  constexpr int slotsz = fd_slot(NS, NXA, NQ, DIM, NB, FUSE);
+  constexpr int slotsz = SMALL ? small_slot(NS, NXA, NQ, DIM, FUSE) : fd_slot(NS, NXA, NQ, DIM, NB, FUSE);
   const int tid = threadIdx.x, nth = blockDim.x;
   for (int t = tid; t < NQ * NQ + 1; t += nth) sW[t] = A.tab[NQ * NQ + t];
   double* const s0 = sm + NQ * NQ + 2;
+  // SMALL: Cfd (Cw for the weak form), face fluxes, line forms, pair numbers, pair values
+  constexpr int NLN = line_count(NQ, DIM), NPR = small_pairs(NQ);
+  double* const sC = s0 + slotsz;
+  double* const sF = sC + NQ * NQ;
+  int* const sForm = (int*)(sF + 2 * NLN * NS);
+  int* const sPair = sForm + NLN;
+  double* const sV = sF + 2 * NLN * NS + (NLN + NPR + 1) / 2;
+  if constexpr (SMALL) {
+    for (int t = tid; t < NQ * NQ; t += nth) {
+      sC[t] = A.tab[(VK == VK_WEAK ? NQ * NQ : 0) + t];
+      const int a = t / NQ, b = t - a * NQ;
+      if (a < b) sPair[a * NQ - a * (a + 1) / 2 + b - a - 1] = a * 16 + b;
+    }
+  }
   // regions of an element's slot
   constexpr int OX = NS * NPL;                       // point values, later the accumulators
   constexpr int OL = OX + NXA * NPL;                 // fused: linear p', H m_z
@@ -546,18 +711,21 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     // rounds of the node loops: the CTA has a thread per line, so their count
     // is a constant and the loads of all rounds are issued before the first
     // is used
-    constexpr int RN = (NQ + DIM - 1) / DIM;
+    constexpr int RN = SMALL ? 1 : (NQ + DIM - 1) / DIM;  // (SMALL: a thread per node)
     constexpr bool RUS = SF == F_RUSANOV && !S::F32;
     // ------------------------------------------------ this thread's line
     // lines ordered by direction, then element: the lanes of a warp mostly
     // share a direction, and the vertical lines (which carry the fused linear
     // operator) fill few warps
     const int nld = E * NFP;
-    const int d = DIM == 3 ? (tid >= nld) + (tid >= 2 * nld) : (tid >= nld);
-    const int es_ = (tid - d * nld) / NFP;
+    // (SMALL: the next NLN threads own the lines' second faces)
+    const int side = SMALL && tid >= NLN;
+    const int tl = side ? tid - NLN : tid;
+    const int d = DIM == 3 ? (tl >= nld) + (tl >= 2 * nld) : (tl >= nld);
+    const int es_ = (tl - d * nld) / NFP;
     const bool line = es_ < ne && tid < DIM * nld;
     const int es = line ? es_ : 0;  // a thread without a line works on the first element and stores nothing
-    const int l = tid < DIM * nld ? tid - d * nld - es_ * NFP : 0;
+    const int l = tl < DIM * nld ? tl - d * nld - es_ * NFP : 0;
     const int e = tile * E + es;
     const bool act = (A.dirs >> d) & 1;
     int rot[DIM];
@@ -568,13 +736,13 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     // are free of branches.
     int nv[2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) nv[i] = __ldg(A.nbr + 6 * e + 2 * d + i);
+    for (int i = 0; i < 2; ++i) nv[i] = __ldg(A.nbr + 6 * e + 2 * d + (SMALL && i == 0 ? side : i));
     const double gd = __ldg(A.ginv + 3 * e + d);
     double qp[2][NS], ap[2];
     size_t nid[2];
     auto face_load = [&](int i) {
       const bool inner = nv[i] > NBR_BOUNDARY + 64;
-      const bool hi = inner != (i == 1);  // the trace lies at the element's last node of the line
+      const bool hi = inner != ((SMALL && i == 0 ? side : i) == 1);  // the trace lies at the element's last node of the line
       nid[i] = (size_t)(e + (inner ? nv[i] : 0)) * NP + line_base<NQ, DIM>(d, l, NQ) +
                (hi ? NQ - 1 : 0) * line_stride<NQ, DIM>(d, NQ);
       qp[i][0] = __ldg(A.q[0] + nid[i]);
@@ -687,6 +855,10 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
     double* const sx = sq + OX;
     const int base = line_base<NQ, DIM>(d, l, ROW), sd = line_stride<NQ, DIM>(d, ROW);
     constexpr bool XYZ = VK == VK_EC32 && !S::SW;  // accumulators in x, y, z order
+    if constexpr (SMALL) {
+      if (tid < NLN) sForm[tid] = line_form<LAW, DIM, VK, NQ>(sq, sx, base, sd);
+      __syncthreads();
+    }
     double T[NQ][NS], X[NQ];
 #pragma unroll
     for (int a = 0; a < NQ; ++a) {
@@ -695,7 +867,8 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
       for (int s = 0; s < NS; ++s) T[a][s] = 0.0;
     }
     if (act) {
-      // ---- the numerical fluxes at the line's ends, one lift_end * flux each
+      // ---- the numerical fluxes at the line's ends, one lift_end * flux each (i: the
+      // end; k: its place in the arrays above)
       auto own = [&](int i, double* qm, double* am) {
         const int nm = base + (i ? (NQ - 1) * sd : 0);
         qm[0] = sq[nm];
@@ -709,19 +882,19 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           if (LAW == LAW_EG && !S::F32) am[0] = 4.0 * am[0];
         }
       };
-      auto bc = [&](int i, const LawP& Lb, const double* qm, double* qb) {
+      auto bc = [&](int k, int i, const LawP& Lb, const double* qm, double* qb) {
         if constexpr (F32S) {
           const int id[3] = {0, 1, 2};
-          boundary_state_rot<LAW, DIM>(Lb, d, id, d, i ? 1.0 : -1.0, nv[i] - NBR_BOUNDARY, qm, qb);
+          boundary_state_rot<LAW, DIM>(Lb, d, id, d, i ? 1.0 : -1.0, nv[k] - NBR_BOUNDARY, qm, qb);
         } else {
-          boundary_state_rot<LAW, DIM>(Lb, d, rot, 0, i ? 1.0 : -1.0, nv[i] - NBR_BOUNDARY, qm, qb);
+          boundary_state_rot<LAW, DIM>(Lb, d, rot, 0, i ? 1.0 : -1.0, nv[k] - NBR_BOUNDARY, qm, qb);
         }
       };
       // pde_level_balance: the reference state too
-      auto aux = [&](int i, double* am, double* apv) {
+      auto aux = [&](int f, int i, double* am, double* apv) {
 #pragma unroll
         for (int k = 0; k < NAM; ++k) apv[k] = 0.0;
-        apv[0] = ap[i];
+        apv[0] = ap[f];
         if (LAW == LAW_EG && (RUS ? L.pde != 0 : A.naux_nl > 1)) {
           const size_t mid = (size_t)e * NP + line_base<NQ, DIM>(d, l, NQ) +
                              (size_t)(i ? (NQ - 1) : 0) * line_stride<NQ, DIM>(d, NQ);
@@ -729,39 +902,66 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           for (int k = 1; k < NAM; ++k)
             if (k < A.naux_nl) {
               am[k] = __ldg(A.aux + k * A.stride + mid);
-              apv[k] = __ldg(A.aux + k * A.stride + nid[i]);
+              apv[k] = __ldg(A.aux + k * A.stride + nid[f]);
             }
         }
       };
-      double qm[2][NS], am[2][NAM], apv[2][NAM], nf[2][NS];
-      // both ends in one stretch of code: their chains overlap
+      if constexpr (SMALL) {
+        if (tid < 2 * NLN) {
+          const double sgn = side ? 1.0 : -1.0;
+          double qm[NS], am[NAM], apv[NAM], nf[NS];
+          own(side, qm, am);
+          if (nv[0] <= NBR_BOUNDARY + 64) bc(0, side, L, qm, qp[0]);
+          aux(0, side, am, apv);
+          if constexpr (RUS)
+            line_rusanov<LAW, DIM>(L, sgn, qm, am, qp[0], apv, nf);
+          else
+            line_flux<LAW, DIM, S::F32, SF>(L, sflux, d, sgn, qm, am, qp[0], apv, nf);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        own(i, qm[i], am[i]);
-        if (nv[i] <= NBR_BOUNDARY + 64) bc(i, L, qm[i], qp[i]);
-        aux(i, am[i], apv[i]);
-      }
+          for (int s = 0; s < NS; ++s) {
+            double f = nf[s];
+            if constexpr (F32S && !XYZ) {  // fluxes in x, y, z order, sums rotated
+              if (s > 0 && s <= DIM) {
+                f = nf[1];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const double sgn = i ? 1.0 : -1.0;
-        if constexpr (RUS)
-          line_rusanov<LAW, DIM>(L, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
-        else
-          line_flux<LAW, DIM, S::F32, SF>(L, sflux, d, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
-      }
+                for (int k = 1; k < DIM; ++k)
+                  if (rot[s - 1] == k) f = nf[1 + k];
+              }
+            }
+            sF[s * 2 * NLN + tid] = __dmul_rn(-lift_end, f);
+          }
+        }
+      } else {
+        double qm[2][NS], am[2][NAM], apv[2][NAM], nf[2][NS];
+        // both ends in one stretch of code: their chains overlap
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        double(&Te)[NS] = T[i ? NQ - 1 : 0];
+        for (int i = 0; i < 2; ++i) {
+          own(i, qm[i], am[i]);
+          if (nv[i] <= NBR_BOUNDARY + 64) bc(i, i, L, qm[i], qp[i]);
+          aux(i, i, am[i], apv[i]);
+        }
 #pragma unroll
-        for (int s = 0; s < NS; ++s) Te[s] = __dmul_rn(-lift_end, nf[i][s]);
-        if constexpr (F32S && !XYZ) {  // fluxes in x, y, z order, accumulators rotated
+        for (int i = 0; i < 2; ++i) {
+          const double sgn = i ? 1.0 : -1.0;
+          if constexpr (RUS)
+            line_rusanov<LAW, DIM>(L, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
+          else
+            line_flux<LAW, DIM, S::F32, SF>(L, sflux, d, sgn, qm[i], am[i], qp[i], apv[i], nf[i]);
+        }
 #pragma unroll
-          for (int c = 0; c < DIM; ++c) {
-            double f = nf[i][1];
+        for (int i = 0; i < 2; ++i) {
+          double(&Te)[NS] = T[i ? NQ - 1 : 0];
 #pragma unroll
-            for (int k = 1; k < DIM; ++k)
-              if (rot[c] == k) f = nf[i][1 + k];
-            Te[1 + c] = __dmul_rn(-lift_end, f);
+          for (int s = 0; s < NS; ++s) Te[s] = __dmul_rn(-lift_end, nf[i][s]);
+          if constexpr (F32S && !XYZ) {  // fluxes in x, y, z order, accumulators rotated
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) {
+              double f = nf[i][1];
+#pragma unroll
+              for (int k = 1; k < DIM; ++k)
+                if (rot[c] == k) f = nf[i][1 + k];
+              Te[1 + c] = __dmul_rn(-lift_end, f);
+            }
           }
         }
       }
@@ -856,30 +1056,120 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         }
       }
     }
-    // the form of the line's logarithmic means: how far apart its densities and
-    // B lie, from the high words (monotonic for positive values; NaN and
-    // non-positive values fail both tests)
     int form = 0;
-    if constexpr ((VK == VK_EC || VK == VK_EC32) && !S::SW) {
-      int rlo = 0x7fffffff, rhi = -0x7fffffff - 1, blo = rlo, bhi = rhi;
+    if constexpr (!SMALL) form = line_form<LAW, DIM, VK, NQ>(sq, sx, base, sd);
+    double Ts[NS];  // SMALL: the node's sums
+    if constexpr (SMALL) {
+      const int n0 = tid < NP ? tid : 0, i0 = n0 % NQ, i1 = n0 / NQ % NQ, i2 = n0 / (NQ * NQ);
+      const int pn = n0 + (ROW - NQ) * (n0 / NQ);
+      constexpr int DB = VK == VK_WEAK ? DIM : small_batch(NQ, DIM), NT = DB * NFP * NPR;
+      const double c0 = (VK == VK_EC && !S::SW) ? 2.0 / (L.gamma - 1.0) : S::SW ? 0.5 * L.grav : 1.0 / (L.gamma - 1.0);
 #pragma unroll
-      for (int a = 0; a < NQ; ++a) {
-        const int n = base + a * sd;
-        const int hr = __double2hiint(sq[n]), hb = __double2hiint(sx[(VK == VK_EC ? DIM : 1) * NPL + n]);
-        rlo = min(rlo, hr);
-        rhi = max(rhi, hr);
-        blo = min(blo, hb);
-        bhi = max(bhi, hb);
+      for (int d0 = 0; d0 < DIM; d0 += DB) {
+        if constexpr (VK != VK_WEAK) {
+          if (d0 > 0) __syncthreads();
+#pragma unroll 1
+          for (int t = tid; t < NT; t += nth) {
+            const int td = t / (NFP * NPR), r = t - td * (NFP * NPR), pi = r / NFP, tln = r - pi * NFP, dd = d0 + td;
+            if (!((A.dirs >> dd) & 1)) continue;
+            int rt[DIM];
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) rt[c] = line_rot<DIM>(c, dd);
+            const int b0 = line_base<NQ, DIM>(dd, tln, ROW), st = line_stride<NQ, DIM>(dd, ROW), ab = sPair[pi];
+            LinePt<LAW, DIM, VK> P, Q;
+            line_load<LAW, DIM, VK, false>(P, sq, sx, NPL, b0 + (ab >> 4) * st, rt, dd);
+            line_load<LAW, DIM, VK, false>(Q, sq, sx, NPL, b0 + (ab & 15) * st, rt, dd);
+            double f[NS], x = 0.0;
+            if constexpr (VK == VK_EC && !S::SW) {
+              const int fo = sForm[dd * NFP + tln];
+              if (fo == 0)
+                line_pair<LAW, DIM, VK, 0>(L, c0, dd, P, Q, f, x);
+              else if (fo == 1)
+                line_pair<LAW, DIM, VK, 1>(L, c0, dd, P, Q, f, x);
+              else
+                line_pair<LAW, DIM, VK, 2>(L, c0, dd, P, Q, f, x);
+            } else if constexpr (VK == VK_EC32 && !S::SW) {
+              if (sForm[dd * NFP + tln] == 0)
+                line_pair<LAW, DIM, VK, 0>(L, c0, dd, P, Q, f, x);
+              else
+                line_pair<LAW, DIM, VK, 2>(L, c0, dd, P, Q, f, x);
+            } else {
+              line_pair<LAW, DIM, VK, 0>(L, c0, dd, P, Q, f, x);
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) sV[s * NT + t] = f[s];
+            if constexpr (S::XTRA) sV[NS * NT + t] = x;
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int dd = d0; dd < d0 + DB && dd < DIM; ++dd) {
+          double t[NS];
+#pragma unroll
+          for (int s = 0; s < NS; ++s) t[s] = 0.0;
+          if (tid < NP && ((A.dirs >> dd) & 1)) {
+            const int a = dd == 0 ? i0 : dd == 1 ? i1 : i2;
+            const int ln = DIM == 2 ? (dd == 0 ? i1 : i0) : dd == 0 ? i1 + NQ * i2 : dd == 1 ? i0 + NQ * i2 : i0 + NQ * i1;
+            if (a == 0 || a == NQ - 1) {
+              const int fc = (a == 0 ? 0 : NLN) + dd * NFP + ln;
+#pragma unroll
+              for (int s = 0; s < NS; ++s) t[s] = sF[s * 2 * NLN + fc];
+            }
+            if constexpr (VK == VK_WEAK) {
+              int rt[DIM];
+#pragma unroll
+              for (int c = 0; c < DIM; ++c) rt[c] = line_rot<DIM>(c, dd);
+              const int b0 = line_base<NQ, DIM>(dd, ln, ROW), st = line_stride<NQ, DIM>(dd, ROW);
+#pragma unroll
+              for (int m = 0; m < NQ; ++m) {
+                double f[NS];
+                weak_row<DIM>(sq, sx, NPL, b0 + m * st, rt, f);
+                const double c = sC[a * NQ + m];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) t[s] = fma(c, f[s], t[s]);
+              }
+            } else {
+              double X = 0.0;
+#pragma unroll
+              for (int b = 0; b < NQ; ++b) {
+                if (b == a) continue;
+                const int lo = b < a ? b : a, hi = b < a ? a : b;
+                const double* const v = sV + ((dd - d0) * NPR + lo * NQ - lo * (lo + 1) / 2 + hi - lo - 1) * NFP + ln;
+                const double c = sC[a * NQ + b];
+                double f[NS];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) f[s] = v[s * NT];
+                if constexpr (S::EG && (VK == VK_KG || VK == VK_KG32)) {
+                  const double x = v[NS * NT];
+                  f[1] = b < a ? f[1] + x : f[1] - x;
+                } else if constexpr (S::XTRA) {
+                  X = fma(b < a ? -c : c, v[NS * NT], X);
+                }
+#pragma unroll
+                for (int s = 0; s < NS; ++s) t[s] = fma(c, f[s], t[s]);
+              }
+              if constexpr (S::XTRA && VK != VK_KG && VK != VK_KG32) {
+                if constexpr (S::SW)
+                  X = L.swtopo ? __dmul_rn(X, 0.5 * L.grav * sq[pn]) : 0.0;
+                else if constexpr (VK == VK_EC)
+                  X = __dmul_rn(X, sx[(DIM + 1) * NPL + pn]);
+                else if constexpr (VK == VK_EC32)
+                  X = __dmul_rn(X, sx[2 * NPL + pn]);
+                t[XYZ ? 1 + dd : 1] -= X;
+              }
+            }
+            const double gn = __ldg(A.ginv + 3 * e + dd);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) t[s] = __dmul_rn(t[s], gn);
+          }
+#pragma unroll
+          for (int s = 0; s < NS; ++s) {
+            const int c = (s == 0 || s == DIM + 1 || XYZ) ? s : 1 + (s - 1 + dd) % DIM;
+            Ts[c] = dd == 0 ? t[s] : Ts[c] + t[s];
+          }
+        }
       }
-      const double rmax = __hiloint2double(rhi + 1, 0), bmax = __hiloint2double(bhi + 1, 0);
-      const double rmin = __hiloint2double(rlo, 0), bmin = __hiloint2double(blo, 0);
-      const bool near = rmax < 1.2 * rmin && bmax < 1.2 * bmin;
-      if constexpr (VK == VK_EC32)
-        form = DIM == 3 && __all_sync(0xffffffffu, near) ? 0 : 2;  // (every lane of the CTA is here)
-      else
-        form = near ? 0 : rmax < 3.0 * rmin && bmax < 3.0 * bmin ? 1 : 2;
-    }
-    if (act) {
+    } else if (act) {
       // ---- two-point fluxes of the line's pairs, or the weak form's rows
       if constexpr (VK == VK_WEAK) {
         line_weak<DIM, NQ>(A, sq, sx, base, sd, rot, T);
@@ -893,8 +1183,8 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
           line_pairs<LAW, DIM, VK, NQ, 2>(A, c0, sq, sx, base, sd, rot, d, T, X);
       } else if constexpr (VK == VK_EC32 && !S::SW) {
         const double c0 = 1.0 / (L.gamma - 1.0);
-        if (DIM == 3 && form == 0)
-          line_pairs<LAW, DIM, VK, NQ, (DIM == 3 ? 0 : 2)>(A, c0, sq, sx, base, sd, rot, d, T, X);
+        if (form == 0)
+          line_pairs<LAW, DIM, VK, NQ, 0>(A, c0, sq, sx, base, sd, rot, d, T, X);
         else
           line_pairs<LAW, DIM, VK, NQ, 2>(A, c0, sq, sx, base, sd, rot, d, T, X);
       } else {
@@ -924,8 +1214,9 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         for (int s = 0; s < NS; ++s) T[a][s] = __dmul_rn(T[a][s], gd);
       }
     }
-    __syncthreads();  // the point values are dead: their region takes the sums
-    if constexpr (NB > 1) {
+    if constexpr (!SMALL) __syncthreads();  // the point values are dead: their region takes the sums
+    if constexpr (SMALL) {
+    } else if constexpr (NB > 1) {
       if (line) {  // (an inactive direction writes its zeros)
         double* const B = d == 0 ? sx : sq + OB + (d - 1) * NS * NPL;
 #pragma unroll
@@ -988,7 +1279,7 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
         }
       }
     }
-    __syncthreads();
+    if constexpr (!SMALL) __syncthreads();
     // ----------------------------------------------------------- epilogue
     const bool cor = L.src == SRC_CORIOLIS && ((A.dirs >> DZ) & 1);
 #pragma unroll
@@ -1001,6 +1292,10 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
       double T[NS], TL[NS];
 #pragma unroll
       for (int s = 0; s < NS; ++s) {
+        if constexpr (SMALL) {
+          T[s] = Ts[s];
+          continue;
+        }
         T[s] = qn[OX + s * NPL];
         if constexpr (NB > 1) {
 #pragma unroll
@@ -1100,14 +1395,26 @@ __global__ void __launch_bounds__(fd_cfg(LAW, DIM, VK, NQ).max_threads, fd_cfg(L
 
 template <int LAW, int DIM, int VK, int NQ, bool FUSE = false, int SF = -1, bool PERSIST = false>
 void fd_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    // on failure the launch below reports the error
-    if (cudaFuncSetAttribute(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-      configured = smem;
+  auto go = [&](auto kernel, size_t* configured) {
+    if (smem > 48 * 1024 && smem > *configured) {
+      // on failure the launch below reports the error
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
+        *configured = smem;
+    }
+    launch_maybe_pdl(kernel, dim3(grid), dim3(block), smem, st, A);
+  };
+  static size_t line_smem = 0;
+  if constexpr (!PERSIST && fd_has_small(LAW, DIM, VK, SF)) {
+    if (A.small) {
+      static size_t small_smem = 0;
+      using S = LineShape<LAW, DIM, VK>;
+      grid = A.K;
+      block = A.small;
+      smem = sizeof(double) * small_doubles(S::NS, S::NXA, NQ, DIM, FUSE, VK != VK_WEAK);
+      return go(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, false, true>, &small_smem);
+    }
   }
-  launch_maybe_pdl(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>, dim3(grid), dim3(block), smem, st, A);
+  go(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>, &line_smem);
 }
 
 // the kernel of a node count (persistent ones: Nq = 4..6)

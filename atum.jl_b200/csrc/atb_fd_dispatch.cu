@@ -11,6 +11,7 @@ tend_launch_fn fd_eg3_ec32_rus(int nq);
 tend_launch_fn fd_eg3_ec32_any(int nq);
 tend_launch_fn fd_eg3_kg_rus(int nq);
 tend_launch_fn fd_eg3_kg_any(int nq);
+tend_launch_fn fd_eg3_kg32_rus(int nq);
 tend_launch_fn fd_eg3_kg32_any(int nq);
 tend_launch_fn fd_eg3_weak_rus(int nq);
 tend_launch_fn fd_eg3_weak_any(int nq);
@@ -25,6 +26,7 @@ tend_launch_fn fd_euler2_ec_any(int nq);
 tend_launch_fn fd_euler2_ec32_any(int nq);
 tend_launch_fn fd_eg2_ec_rus(int nq);
 tend_launch_fn fd_eg2_ec_any(int nq);
+tend_launch_fn fd_eg2_ec32_rus(int nq);
 tend_launch_fn fd_eg2_ec32_any(int nq);
 tend_launch_fn fd_sw2_ec_rus(int nq);
 tend_launch_fn fd_sw2_ec32_rus(int nq);
@@ -42,12 +44,12 @@ tend_launch_fn pick_fd(int law, int dim, int vk, int nq, int sflux) {
     if (vk == VK_EC) return rus ? fd_eg3_ec_rus(nq) : fd_eg3_ec_any(nq);
     if (vk == VK_EC32) return rus ? fd_eg3_ec32_rus(nq) : fd_eg3_ec32_any(nq);
     if (vk == VK_KG) return rus ? fd_eg3_kg_rus(nq) : fd_eg3_kg_any(nq);
-    if (vk == VK_KG32) return fd_eg3_kg32_any(nq);
+    if (vk == VK_KG32) return rus ? fd_eg3_kg32_rus(nq) : fd_eg3_kg32_any(nq);
     if (vk == VK_WEAK) return rus ? fd_eg3_weak_rus(nq) : fd_eg3_weak_any(nq);
   }
   if (law == LAW_EG && dim == 2) {
     if (vk == VK_EC) return rus ? fd_eg2_ec_rus(nq) : fd_eg2_ec_any(nq);
-    if (vk == VK_EC32) return fd_eg2_ec32_any(nq);
+    if (vk == VK_EC32) return rus ? fd_eg2_ec32_rus(nq) : fd_eg2_ec32_any(nq);
   }
   if (law == LAW_EULER && dim == 3 && vk == VK_EC) return fd_euler3_ec_any(nq);
   if (law == LAW_EULER && dim == 2) {

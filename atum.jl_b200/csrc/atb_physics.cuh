@@ -143,6 +143,19 @@ static __device__ __noinline__ double logavg_wide(double a, double b) {
   return (a - b) / log(a / b);
 }
 
+// 1/d in FP32 for normal d, and n / d from it by Markstein's theorem (Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990): one correction
+// of the quotient by its exact residual rounds as the division does
+__device__ __forceinline__ float rcp32(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return fmaf(fmaf(-d, r, 1.f), r, r);
+}
+__device__ __forceinline__ float div32(float n, float d, float r) {
+  const float q = __fmul_rn(n, r);
+  return fmaf(fmaf(-d, q, n), r, q);
+}
+
 template <class T> __device__ __forceinline__ T roe_avg(T srm, T srp, T sm, T sp) {
   return (srm * sm + srp * sp) / (srm + srp);
 }
@@ -516,9 +529,7 @@ template <class T> __device__ __forceinline__ T series_G(T u) {
 // series correction, so the hydrostatic balance between the pressure and
 // gravity terms is carried in FP64 while every division, logarithm and
 // advective product is FP32.  Returns FP64 row values and b_avg * rho_log.
-// NEAR: the caller knows that both logarithmic means of every pair it
-// evaluates are on their series branch (the same values, no branch per pair).
-template <int LAW, int DIM, bool NEAR = false>
+template <int LAW, int DIM>
 __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1, double b1, const float* u1,
                                          float uu1, double Phi1, double r2, double p2, double b2,
                                          const float* u2, float uu2, double Phi2, double* f, double* xtra) {
@@ -529,7 +540,7 @@ __device__ __forceinline__ void ec_vol32(float igm1, int d, double r1, double p1
   const float ur = fr * fr, ub = fb * fb;
   double rho_log;
   float cterm;
-  if (NEAR || (ur < 1e-2f && ub < 1e-2f)) {
+  if (ur < 1e-2f && ub < 1e-2f) {
     // 1 - G(u) = u/3 + 4u^2/45 + 44u^3/945 + ... (the terms of series_G)
     const float cr = ur * (1.f / 3.f + ur * (4.f / 45.f + ur * (44.f / 945.f + ur * (428.f / 14175.f +
                      ur * (10196.f / 467775.f + ur * (10719068.f / 638512875.f + ur * (25865068.f / 1915538625.f)))))));

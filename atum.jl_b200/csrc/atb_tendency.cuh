@@ -67,6 +67,7 @@ struct TendArgs {
   double cfd[64];      // Cfd again for the flux-differencing kernels (Nq <= 8): constant-bank operands
   LawP law;
   int dirs, sflux, epi;
+  int small;           // line kernels: threads of the mode for grids of one wave, or 0 (atb_fd.cuh)
   double a, bdt;
   const double* dte;  // per-element time step (batched instances), or null
   // EPI_ARK accumulators (acc[j][0] null: inactive; accin[j][0] null: base Q)
