@@ -406,9 +406,10 @@ __global__ void __launch_bounds__(curved_fd_cfg(NQ).max_threads, curved_fd_cfg(N
       const double rmax = __hiloint2double(rhi + 1, 0), bmax = __hiloint2double(bhi + 1, 0);
       const double rmin = __hiloint2double(rlo, 0), bmin = __hiloint2double(blo, 0);
       const double c0 = 2.0 / (L.gamma - 1.0);
-      if (rmax < 1.2 * rmin && bmax < 1.2 * bmin)
+      const bool plain = min(rlo, blo) >= ((1023 - 240) << 20) && max(rhi, bhi) < ((1023 + 240) << 20);
+      if (plain && rmax < 1.2 * rmin && bmax < 1.2 * bmin)
         curved_pairs<LAW, VK, NQ, 0>(A, c0, sq, sx, base, sd, d, T);
-      else if (rmax < 3.0 * rmin && bmax < 3.0 * bmin)
+      else if (plain && rmax < 3.0 * rmin && bmax < 3.0 * bmin)
         curved_pairs<LAW, VK, NQ, 1>(A, c0, sq, sx, base, sd, d, T);
       else
         curved_pairs<LAW, VK, NQ, 2>(A, c0, sq, sx, base, sd, d, T);
