@@ -32,7 +32,7 @@ def nvcc() -> str:
 
 
 def _newest_header() -> float:
-    hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    hs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.hpp")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
     return max((os.path.getmtime(h) for h in hs), default=0.0)
 
 

@@ -204,12 +204,8 @@ typedef void (*solve_fn)(const BandSolve&, cudaStream_t);
 template <int NQ, int NS> void solve_launch(const BandSolve& B, cudaStream_t st) {
   constexpr int LPB = 32;
   constexpr size_t smem = sizeof(double) * 2 * (NQ * NS) * (2 * NQ * NS);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    cudaFuncSetAttribute(band_solve_shared_kernel<NQ, NS, LPB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-  }
-  configured = true;
+  static SmemLimit limit;
+  raise_smem(band_solve_shared_kernel<NQ, NS, LPB>, limit, smem);
   band_solve_shared_kernel<NQ, NS, LPB><<<(B.M.nlines + LPB - 1) / LPB, LPB, smem, st>>>(B);
 }
 
@@ -343,10 +339,8 @@ void rows_launch(const BandSolve& B, cudaStream_t st) {
   constexpr int BW1 = NQ * NS;
   constexpr int LPB = 16;
   constexpr size_t smem = sizeof(double) * (4 * BW1 * BW1 + 3 * BW1 * LPB);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024)
-    cudaFuncSetAttribute(band_solve_rows_kernel<NQ, NS, LPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  configured = true;
+  static SmemLimit limit;
+  raise_smem(band_solve_rows_kernel<NQ, NS, LPB>, limit, smem);
   band_solve_rows_kernel<NQ, NS, LPB><<<(B.M.nlines + LPB - 1) / LPB, BW1 * LPB, smem, st>>>(B, B.blk);
 }
 
@@ -591,11 +585,8 @@ void mma_launch(const BandSolve& B, cudaStream_t st) {
   constexpr int NTH = 32 * ((BW1 + 7) / 8);
   static_assert(NQ * LPC <= NTH, "the right-hand-side loader needs NQ*LPC threads");
   constexpr size_t smem = sizeof(double) * (4 * KP * (LPC + 4) + D * 5 * NS * NQ * LPC);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024)
-    cudaFuncSetAttribute(band_solve_mma_kernel<NQ, NS, NT, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-  configured = true;
+  static SmemLimit limit;
+  raise_smem(band_solve_mma_kernel<NQ, NS, NT, D>, limit, smem);
   band_solve_mma_kernel<NQ, NS, NT, D><<<(B.M.nlines + LPC - 1) / LPC, NTH, smem, st>>>(B, B.blk);
 }
 
@@ -932,10 +923,8 @@ constexpr size_t kWarpSolveSmemMax = 227 * 1024;
 template <int NQ, int NS, int NW, int H>
 void warp_launch_nw(const BandSolve& B, cudaStream_t st) {
   constexpr size_t smem = warp_solve_smem<NQ, NS, NW>();
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024)
-    cudaFuncSetAttribute(band_solve_warp_kernel<NQ, NS, NW, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  configured = true;
+  static SmemLimit limit;
+  raise_smem(band_solve_warp_kernel<NQ, NS, NW, H>, limit, smem);
   const int warps = (B.M.nlines + 7) / 8;
   launch_maybe_pdl(band_solve_warp_kernel<NQ, NS, NW, H>, dim3((warps + NW - 1) / NW),
                    dim3(32 * NW * H), smem, st, B);

@@ -258,12 +258,8 @@ __global__ void __launch_bounds__(512) curved_kernel(const TendArgs A) {
 
 template <int LAW, int VK, int SF>
 void curved_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    if (cudaFuncSetAttribute(curved_kernel<LAW, VK, SF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-        cudaSuccess)
-      configured = smem;
-  }
+  static SmemLimit limit;
+  raise_smem(curved_kernel<LAW, VK, SF>, limit, smem);
   launch_maybe_pdl(curved_kernel<LAW, VK, SF>, dim3(grid), dim3(block), smem, st, A);
 }
 

@@ -519,13 +519,8 @@ __global__ void __launch_bounds__(curved_fd_cfg(NQ).max_threads, curved_fd_cfg(N
 
 template <int LAW, int VK, int NQ, bool FUSE, int SF>
 void curved_fd_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    // on failure the launch below reports the error
-    if (cudaFuncSetAttribute(curved_fd_kernel<LAW, VK, NQ, FUSE, SF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) == cudaSuccess)
-      configured = smem;
-  }
+  static SmemLimit limit;
+  raise_smem(curved_fd_kernel<LAW, VK, NQ, FUSE, SF>, limit, smem);
   launch_maybe_pdl(curved_fd_kernel<LAW, VK, NQ, FUSE, SF>, dim3(grid), dim3(block), smem, st, A);
 }
 

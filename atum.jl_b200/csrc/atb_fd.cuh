@@ -1397,26 +1397,20 @@ __global__ void __launch_bounds__(SMALL ? small_threads(NQ, DIM) : fd_cfg(LAW, D
 
 template <int LAW, int DIM, int VK, int NQ, bool FUSE = false, int SF = -1, bool PERSIST = false>
 void fd_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
-  auto go = [&](auto kernel, size_t* configured) {
-    if (smem > 48 * 1024 && smem > *configured) {
-      // on failure the launch below reports the error
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-        *configured = smem;
-    }
-    launch_maybe_pdl(kernel, dim3(grid), dim3(block), smem, st, A);
-  };
-  static size_t line_smem = 0;
   if constexpr (!PERSIST && fd_has_small(LAW, DIM, VK, SF)) {
     if (A.small) {
-      static size_t small_smem = 0;
       using S = LineShape<LAW, DIM, VK>;
-      grid = A.K;
-      block = A.small;
-      smem = sizeof(double) * small_doubles(S::NS, S::NXA, NQ, DIM, FUSE, VK != VK_WEAK);
-      return go(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, false, true>, &small_smem);
+      constexpr size_t bytes =
+          sizeof(double) * small_doubles(S::NS, S::NXA, NQ, DIM, FUSE, VK != VK_WEAK);
+      static SmemLimit small_limit;
+      raise_smem(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, false, true>, small_limit, bytes);
+      launch_maybe_pdl(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, false, true>, dim3(A.K), dim3(A.small), bytes, st, A);
+      return;
     }
   }
-  go(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>, &line_smem);
+  static SmemLimit limit;
+  raise_smem(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>, limit, smem);
+  launch_maybe_pdl(fd_kernel<LAW, DIM, VK, NQ, FUSE, SF, PERSIST>, dim3(grid), dim3(block), smem, st, A);
 }
 
 // the kernel of a node count (persistent ones: Nq = 4..6)

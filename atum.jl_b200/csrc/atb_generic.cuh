@@ -2,6 +2,7 @@
 // banded operator (probe assembly, no-pivot LU, batched solve fused with the
 // ARK right-hand-side combination), reduction finalisation and the FP64 probe.
 #pragma once
+#include "atb_smem.hpp"
 #include <cuda_runtime.h>
 #include <stddef.h>
 
@@ -129,6 +130,17 @@ cudaError_t launch_maybe_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+// raises the kernel's dynamic shared memory limit on the current device where the
+// launch needs it; on failure the launch reports the error
+template <class Kernel> void raise_smem(Kernel* kernel, SmemLimit& limit, size_t smem) {
+  if (smem <= SmemLimit::kDefault) return;
+  int dev = -1;
+  cudaGetDevice(&dev);
+  limit.raise(dev, smem, [&] {
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
 }
 
 }  // namespace atb

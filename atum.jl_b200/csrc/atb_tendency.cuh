@@ -638,13 +638,8 @@ typedef void (*tend_launch_fn)(const TendArgs& A, int grid, int block, size_t sm
 
 template <int LAW, int DIM, int VK, int NQ_ = 0>
 void tend_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream_t st) {
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    // on failure the launch below reports the error
-    if (cudaFuncSetAttribute(tendency_kernel<LAW, DIM, VK, NQ_>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-      configured = smem;
-  }
+  static SmemLimit limit;
+  raise_smem(tendency_kernel<LAW, DIM, VK, NQ_>, limit, smem);
   launch_maybe_pdl(tendency_kernel<LAW, DIM, VK, NQ_>, dim3(grid), dim3(block), smem, st, A);
 }
 
