@@ -1105,7 +1105,7 @@ struct atb_solver {
   // operator), when the two operators allow it (atb_solver_fuse)
   tend_launch_fn fused = nullptr;
   bool fuse_on = false;
-  int lines_sparse = 0;  // band: the stream of nonzero entries of per-line factors (launch_line_stream)
+  int lines = LINES_BAND;  // what band holds for per-line factors
   // per-element time steps (LSRK over packed instances), or null; owned by
   // the solver (atb_solver_set_instance_dt) or by the caller
   double* d_dte = nullptr;
@@ -1277,7 +1277,8 @@ int build_band(atb_solver* s, cudaStream_t st) {
     launch_band_factor(M.nunk, M.bw, M.nlines, s->band, W, M.nlines, scale, st);
     s->ld = M.nlines;
     // the face-node coupling structure of every line's factor lets the solve
-    // leave the zero blocks out (ATB_BAND_DENSE=1 keeps the full band)
+    // leave the zero blocks out (ATB_BAND_DENSE=1 reads the full band,
+    // ATB_BAND_DENSE=2 the band without its zero blocks)
     int* d_bad = nullptr;
     if ((rc = dalloc(&d_bad, 1))) return rc;
     CK(cudaMemsetAsync(d_bad, 0, sizeof(int), st));
@@ -1290,16 +1291,18 @@ int build_band(atb_solver* s, cudaStream_t st) {
     const size_t sn = line_stream_doubles(M);
     if (bad == 0 && sn > 0 && !(dense && dense[0] == '1')) {
       // the nonzero entries as each warp's stream instead of the band; without
-      // the memory to hold both for a moment the solve reads the band
+      // the memory to hold both for a moment the solve reads them from the band
+      s->lines = LINES_FACES;
       double* stream = nullptr;
-      if (cudaMalloc(&stream, sn * sizeof(double)) == cudaSuccess) {
+      if (dense && dense[0] == '2') {
+      } else if (cudaMalloc(&stream, sn * sizeof(double)) == cudaSuccess) {
         if (launch_line_stream(M, s->band, stream, st) != cudaSuccess) {
           cudaFree(stream);
           return fail(ATB_ERR_CUDA, "laying out the band factor failed");
         }
         cudaFree(s->band);
         s->band = stream;
-        s->lines_sparse = 1;
+        s->lines = LINES_STREAM;
       } else {
         cudaGetLastError();  // the failed allocation is not the caller's error
       }
@@ -1588,7 +1591,7 @@ int ark_step_accumulated(atb_solver* s, double* const* q, cudaStream_t st) {
     B.blk = s->blk;
     B.frag = s->frag;
     B.ld = s->ld;
-    B.lines_sparse = s->lines_sparse;
+    B.lines = s->lines;
     B.npairs = 0;
     B.dt = s->dt;
     for (int c = 0; c < 5; ++c) { B.q[c] = R[c]; B.out[c] = Qout[c]; }
@@ -1680,7 +1683,7 @@ int ark_step(atb_solver* s, double* const* q, cudaStream_t st) {
       B.blk = s->blk;
       B.frag = s->frag;
       B.ld = s->ld;
-      B.lines_sparse = s->lines_sparse;
+      B.lines = s->lines;
       B.npairs = i;
       B.dt = s->dt;
       for (int k = 0; k < i; ++k) {
@@ -1862,6 +1865,10 @@ extern "C" int atb_solve(atb_solver* s, double* const* q, double timeend, int ad
   if (steps_out) *steps_out = step;
   return ATB_OK;
 }
+
+// what the solver's per-line factors are held as (LINES_*), -1 without such factors;
+// for the tests (not part of the C ABI's header)
+extern "C" int atb_detail_solver_lines(const atb_solver* s) { return s && s->band && s->ld > 1 ? s->lines : -1; }
 
 extern "C" int atb_solver_get(const atb_solver* s, double* time, double* dt, double* gamma) {
   if (!s) return fail(ATB_ERR_INVALID, "null solver");

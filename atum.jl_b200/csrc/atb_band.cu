@@ -1084,12 +1084,12 @@ namespace {
 // is read before the wait); a ring of 5 such chunks 164 us.
 //
 // band_solve_lines_kernel: any band, the factor in the line-fastest layout
-// band[(r * W + k) * nlines + line]; for coupling structures other than the
-// above.
-
+// band[(r * W + k) * nlines + line], for other coupling structures; SPARSE leaves
+// out the entries that the face-node structure makes zero (half of the bytes),
+// where there was no memory to lay out the stream beside the band.
 // one row of the forward (FWD) or backward pass, then the next: compile-time
 // row indices keep every block value in a register
-template <int NQ, int NS, bool FWD, int I>
+template <int NQ, int NS, bool SPARSE, bool FWD, int I>
 __device__ __forceinline__ void lines_rows(const BandSolve& B, const double* __restrict__ row0, size_t ld,
                                            size_t eoff, int nh, bool has_nb, const double (&nb)[NQ * NS],
                                            double (&cur)[NQ * NS]) {
@@ -1107,29 +1107,35 @@ __device__ __forceinline__ void lines_rows(const BandSolve& B, const double* __r
         if (k < B.npairs) acc = acc + B.dt * (B.a[k] * B.ex[k][s][g] + B.b[k] * B.im[k][s][g]);
       if (has_nb) {
 #pragma unroll
-        for (int jp = I + 1; jp < BW1; ++jp) acc = acc - row[(size_t)(jp - I - 1) * ld] * nb[jp];
+        for (int jp = I + 1; jp < BW1; ++jp) {
+          if (SPARSE && !(I < NS && jp >= BW1 - NS)) continue;
+          acc = acc - row[(size_t)(jp - I - 1) * ld] * nb[jp];
+        }
       }
 #pragma unroll
       for (int jp = 0; jp < I; ++jp) acc = acc - row[(size_t)(jp - I + BW) * ld] * cur[jp];
       cur[I] = acc;
       B.out[s][g] = acc;
-      lines_rows<NQ, NS, FWD, I + 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
+      lines_rows<NQ, NS, SPARSE, FWD, I + 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
     } else {
       double acc = B.out[s][g];
 #pragma unroll
       for (int jp = I + 1; jp < BW1; ++jp) acc = acc - row[(size_t)(jp - I + BW) * ld] * cur[jp];
       if (has_nb) {
 #pragma unroll
-        for (int jp = 0; jp < I; ++jp) acc = acc - row[(size_t)(2 * BW1 - 1 + jp - I) * ld] * nb[jp];
+        for (int jp = 0; jp < I; ++jp) {
+          if (SPARSE && !(I >= BW1 - NS && jp < NS)) continue;
+          acc = acc - row[(size_t)(2 * BW1 - 1 + jp - I) * ld] * nb[jp];
+        }
       }
       cur[I] = acc / row[(size_t)BW * ld];
       B.out[s][g] = cur[I];
-      lines_rows<NQ, NS, FWD, I - 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
+      lines_rows<NQ, NS, SPARSE, FWD, I - 1>(B, row0, ld, eoff, nh, has_nb, nb, cur);
     }
   }
 }
 
-template <int NQ, int NS>
+template <int NQ, int NS, bool SPARSE>
 __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B) {
   constexpr int BW1 = NQ * NS;
   constexpr int BW = BW1 - 1;
@@ -1151,7 +1157,7 @@ __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B)
   // forward: L y = rhs (unit diagonal)
   for (int ev = 0; ev < KV; ++ev) {
     const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
-    lines_rows<NQ, NS, true, 0>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev > 0, nb, cur);
+    lines_rows<NQ, NS, SPARSE, true, 0>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev > 0, nb, cur);
 #pragma unroll
     for (int j = 0; j < BW1; ++j) nb[j] = cur[j];
   }
@@ -1160,7 +1166,8 @@ __global__ void __launch_bounds__(64) band_solve_lines_kernel(const BandSolve B)
   for (int j = 0; j < BW1; ++j) nb[j] = 0.0;
   for (int ev = KV - 1; ev >= 0; --ev) {
     const size_t eoff = (size_t)(e0 + ev * M.estep) * Np + hn;
-    lines_rows<NQ, NS, false, BW1 - 1>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev < KV - 1, nb, cur);
+    lines_rows<NQ, NS, SPARSE, false, BW1 - 1>(B, band + (size_t)ev * BW1 * W * ld, ld, eoff, nh, ev < KV - 1, nb,
+                                               cur);
 #pragma unroll
     for (int j = 0; j < BW1; ++j) nb[j] = cur[j];
   }
@@ -1348,10 +1355,13 @@ __global__ void __launch_bounds__(32) band_solve_stream_kernel(const BandSolve B
 
 typedef void (*lines_fn)(const BandSolve& B, cudaStream_t st);
 template <int NQ, int NS> void lines_launch(const BandSolve& B, cudaStream_t st) {
-  if (B.lines_sparse)
+  const dim3 grid((B.M.nlines + 63) / 64);
+  if (B.lines == LINES_STREAM)
     launch_maybe_pdl(band_solve_stream_kernel<NQ, NS>, dim3((B.M.nlines + 31) / 32), dim3(32), 0, st, B);
+  else if (B.lines == LINES_FACES)
+    launch_maybe_pdl(band_solve_lines_kernel<NQ, NS, true>, grid, dim3(64), 0, st, B);
   else
-    launch_maybe_pdl(band_solve_lines_kernel<NQ, NS>, dim3((B.M.nlines + 63) / 64), dim3(64), 0, st, B);
+    launch_maybe_pdl(band_solve_lines_kernel<NQ, NS, false>, grid, dim3(64), 0, st, B);
 }
 template <int NS> lines_fn pick_lines(int nq) {
   switch (nq) {

@@ -74,11 +74,12 @@ struct BandSolve {
   double* out[5];
   const double* blk;  // per-element [L^-1 | G | U^-1 | H] blocks (shared factor), or null
   const double* frag; // the same blocks in matrix-unit fragment order (launch_frag_prep), or null
-  // per-line factors (ld = nlines): 1 when every line's factor couples
-  // neighbouring elements through face nodes only (launch_band_lines_structure)
-  // and band holds the stream of nonzero entries (launch_line_stream)
-  int lines_sparse;
+  int lines;  // per-line factors (ld = nlines): LINES_BAND, LINES_FACES, LINES_STREAM
 };
+// what `band` holds for per-line factors: the full band; the band, whose blocks couple
+// neighbouring elements through face nodes only (launch_band_lines_structure); the
+// stream of the nonzero entries of such factors (launch_line_stream)
+enum { LINES_BAND = 0, LINES_FACES = 1, LINES_STREAM = 2 };
 void launch_band_solve(const BandSolve& B, cudaStream_t st);
 // number of entries of the per-line factors (ld = nlines) outside the
 // face-node coupling structure that are not zero, added to *count
