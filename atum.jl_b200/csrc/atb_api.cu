@@ -28,11 +28,6 @@ template <> tend_launch_fn pick_launcher<LAW_EULER>(int, int);
 template <> tend_launch_fn pick_launcher<LAW_EG>(int, int);
 template <> tend_launch_fn pick_launcher<LAW_LEG>(int, int);
 template <> tend_launch_fn pick_launcher<LAW_SW>(int, int);
-template <> tend_launch_fn pick_launcher_nq<LAW_ADV>(int, int, int);
-template <> tend_launch_fn pick_launcher_nq<LAW_EULER>(int, int, int);
-template <> tend_launch_fn pick_launcher_nq<LAW_EG>(int, int, int);
-template <> tend_launch_fn pick_launcher_nq<LAW_LEG>(int, int, int);
-template <> tend_launch_fn pick_launcher_nq<LAW_SW>(int, int, int);
 template <> red_launch_fn pick_reducer<LAW_ADV>(int);
 template <> red_launch_fn pick_reducer<LAW_EULER>(int);
 template <> red_launch_fn pick_reducer<LAW_EG>(int);
@@ -248,7 +243,6 @@ void fill_args(const atb_op* op, TendArgs& A) {
   A.lin_law = LawP{};
   A.lin_sflux = 0;
   A.lin_gg1 = 0.0;
-  A.lin_dirs = 0;
   A.naux_nl = op->naux_used;
   A.Dmat = op->d_D;
   A.G = op->d_G;
@@ -506,23 +500,24 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
     return fail(ATB_ERR_INVALID,
                 "the FP32-flux form exists for the flux-differencing volume term with the entropy-conservative "
                 "flux (Euler, Euler-gravity, shallow water) or the Kennedy-Gruber flux (Euler, Euler-gravity)");
-  tend_launch_fn fn = nullptr;
+  // the line-per-thread kernel where one is compiled; else the node-per-thread one
+  // (linear Euler-gravity's weak form at a compile-time node count)
+  const int nq = d->N + 1, sf = d->surface_flux;
+  const tend_launch_fn fl = pick_fd(d->law, d->dim, vk, nq, sf);
+  tend_launch_fn fn = fl;
   red_launch_fn rf = nullptr;
-  // a compile-time node-count specialisation when one exists, else the
-  // runtime-Nq kernel
-  const int nq = d->N + 1;
   switch (d->law) {
-    case LAW_ADV: fn = pick_launcher_nq<LAW_ADV>(d->dim, vk, nq); if (!fn) fn = pick_launcher<LAW_ADV>(d->dim, vk); rf = pick_reducer<LAW_ADV>(d->dim); break;
-    case LAW_EULER: fn = pick_launcher_nq<LAW_EULER>(d->dim, vk, nq); if (!fn) fn = pick_launcher<LAW_EULER>(d->dim, vk); rf = pick_reducer<LAW_EULER>(d->dim); break;
-    case LAW_EG: fn = pick_launcher_nq<LAW_EG>(d->dim, vk, nq); if (!fn) fn = pick_launcher<LAW_EG>(d->dim, vk); rf = pick_reducer<LAW_EG>(d->dim); break;
-    case LAW_LEG: fn = pick_launcher_nq<LAW_LEG>(d->dim, vk, nq); if (!fn) fn = pick_launcher<LAW_LEG>(d->dim, vk); rf = pick_reducer<LAW_LEG>(d->dim); break;
-    case LAW_SW: fn = pick_launcher_nq<LAW_SW>(d->dim, vk, nq); if (!fn) fn = pick_launcher<LAW_SW>(d->dim, vk); rf = pick_reducer<LAW_SW>(d->dim); break;
+    case LAW_ADV: if (!fn) fn = pick_launcher<LAW_ADV>(d->dim, vk); rf = pick_reducer<LAW_ADV>(d->dim); break;
+    case LAW_EULER: if (!fn) fn = pick_launcher<LAW_EULER>(d->dim, vk); rf = pick_reducer<LAW_EULER>(d->dim); break;
+    case LAW_EG: if (!fn) fn = pick_launcher<LAW_EG>(d->dim, vk); rf = pick_reducer<LAW_EG>(d->dim); break;
+    case LAW_LEG:
+      fn = pick_launcher_leg_nq(d->dim, vk, nq);
+      if (!fn) fn = pick_launcher<LAW_LEG>(d->dim, vk);
+      rf = pick_reducer<LAW_LEG>(d->dim);
+      break;
+    case LAW_SW: if (!fn) fn = pick_launcher<LAW_SW>(d->dim, vk); rf = pick_reducer<LAW_SW>(d->dim); break;
   }
   if (!fn) return fail(ATB_ERR_INVALID, "unsupported (law %d, volume flux %d) combination", d->law, d->volume_flux);
-  const int sf = d->surface_flux;
-  // the line-per-thread kernel, where one is compiled
-  const tend_launch_fn fl = pick_fd(d->law, d->dim, vk, nq, sf);
-  if (fl) fn = fl;
   bool sf_ok = sf == ATB_FLUX_CENTRAL || sf == ATB_FLUX_RUSANOV;
   if (d->law == LAW_EULER || d->law == LAW_EG) sf_ok = sf_ok || (sf >= ATB_FLUX_EC && sf <= ATB_FLUX_MATRIX);
   if (d->law == LAW_SW) sf_ok = sf_ok || sf == ATB_FLUX_EC || sf == ATB_FLUX_ROE;
@@ -1514,8 +1509,6 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
   atb_op* op = s->rhs;
   TendArgs A;
   fill_args(op, A);
-  const int naux = op->dim + 3;  // [Phi, grad Phi, rho_ref, p_ref] staged for both operators
-  A.naux = naux;
   int E = op_elements(op);
   auto bytes = [&](int e) { return fd_bytes(op, e, true); };
   const size_t share =
@@ -1526,7 +1519,6 @@ int run_fused(atb_solver* s, double* const* Q, const ArkAcc& ark, cudaStream_t s
   A.lin_law = s->lin->law;
   A.lin_gg1 = A.lin_law.gamma / (A.lin_law.gamma - 1.0);
   A.lin_sflux = s->lin->sflux;
-  A.lin_dirs = s->lin->dirs;
   for (int j = 0; j < 3; ++j) {
     for (int c = 0; c < 5; ++c) { A.acc[j][c] = ark.acc[j][c]; A.accin[j][c] = ark.accin[j][c]; }
     A.ca[j] = ark.ca[j];

@@ -74,10 +74,10 @@ struct TendArgs {
   double* acc[3][5];
   const double* accin[3][5];
   double ca[3], cb[3], adt;
-  // fused linear operator (atb_fd.cuh): the linear Euler-gravity law, its
-  // surface flux and directions
+  // fused linear operator (atb_fd.cuh): the linear Euler-gravity law and its
+  // surface flux
   LawP lin_law;
-  int lin_sflux, lin_dirs;
+  int lin_sflux;
   double lin_gg1;  // gamma / (gamma - 1) of the linear law
   int naux_nl;  // aux components the explicit operator's faces read
   size_t stride;      // K*Np
@@ -646,7 +646,7 @@ void tend_launch(const TendArgs& A, int grid, int block, size_t smem, cudaStream
 // generic (runtime Nq) launcher, and the compile-time-Nq specialisations
 // that exist for (law, dim, vk, nq) -- nullptr when there is none
 template <int LAW> tend_launch_fn pick_launcher(int dim, int vk);
-template <int LAW> tend_launch_fn pick_launcher_nq(int dim, int vk, int nq);
+tend_launch_fn pick_launcher_leg_nq(int dim, int vk, int nq);  // linear Euler-gravity
 
 // per-node precomputed values and per-pair stored values, for the host
 inline int npre_of(int law, int dim, int vk) {
