@@ -629,7 +629,8 @@ int op_create_impl(const atb_op_desc* descs, int n, const double* const* aux_hos
     op->fd = true;
     // Cfd, or Cw for the weak form
     std::copy_n(tab.begin() + (vk == VK_WEAK ? Nq * Nq : 0), Nq * Nq, op->cfd);
-    op->E = fd_default_elements(Nq, dim, fd_limit(op), K, nsm, false);
+    op->E = fd_default_elements(Nq, dim, fd_limit(op), K, nsm,
+                                sf == F_RUSANOV || (vk != VK_EC32 && vk != VK_KG32));
     op->small = fd_small(d->law, dim, vk, Nq, sf, K, nsm);
   }
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
@@ -756,7 +757,7 @@ extern "C" int atb_op_create_curved(const atb_op_desc* d, const double* aux_host
   if (d->law == LAW_EG) nu = d->pde_level_balance ? 6 : (op->vk == VK_WEAK ? 4 : 1);
   if (d->law == LAW_LEG) nu = 6;
   op->naux_used = std::min(nu, op->naux);
-  op->E = fd ? fd_default_elements(Nq, 3, fd_limit(op), K, op->nsm, true) : std::max(1, 128 / Np);
+  op->E = fd ? fd_default_elements(Nq, 3, fd_limit(op), K, op->nsm, false) : std::max(1, 128 / Np);
   while (op->E > 1 && op_smem(op, op->E) > 100 * 1024) --op->E;
   op->smem = op_smem(op, op->E);
   if (op->smem > 227 * 1024 || (!fd && cta_threads(op->E, Np) > 512)) {

@@ -1,7 +1,7 @@
 // Flux-differencing tendency kernel, one thread per tensor line.  (Measured on
 // B200 against the node-per-thread form that stored every pair in shared
-// memory: 16^3 elements at N = 4, fused ARK23 stage 88.5 -> 44 us; 32^3 at
-// N = 7, 5.11 -> 1.66 ms; 128 shallow-water basins of 32^2 at N = 4, FP32
+// memory: 16^3 elements at N = 4, fused ARK23 stage 88 -> 52 us by events around
+// each launch (80 -> 44 by difference from the step); 32^3 at N = 7, 5.11 -> 1.66 ms; 128 shallow-water basins of 32^2 at N = 4, FP32
 // flux, 267 -> 114 us per LSRK stage; weak form, 24^3 at N = 4: 206 -> 76 us.)
 //
 // The same stage as atb_tendency.cuh's kernel (volume term, surface term,
@@ -88,8 +88,8 @@ __host__ __device__ constexpr int line_nodes(int nq, int dim) { return line_row(
 // direction writes its own, one barrier) or one that the directions add into in
 // turn.  Measured per order on B200: more warps pay until the spills they force
 // cost more (3-D, Nq = 6: 718 us per LSRK54 step of 20^3 elements at 4 CTAs of
-// 128 threads, 750 at 2 of 224; Nq = 5 fused stage: 44 us at 3 CTAs of 160
-// threads, 49 at 2, 74 at 4); one accumulator array pays where shared memory
+// 128 threads, 750 at 2 of 224; Nq = 5 fused stage, by difference
+// from the step: 44 us at 3 CTAs of 160 threads, 49 at 2, 74 at 4); one accumulator array pays where shared memory
 // or the FP32-flux form's registers limit the CTAs (shallow water, Nq = 5:
 // 561 against 612 us).
 struct FdCfg {
@@ -97,7 +97,10 @@ struct FdCfg {
 };
 __host__ __device__ constexpr FdCfg fd_cfg(int law, int dim, int vk, int nq) {
   const bool f32 = vk == VK_EC32 || vk == VK_KG32;
-  if (dim == 2) return law == LAW_SW ? FdCfg{160, nq <= 5 ? 4 : 3, 1} : FdCfg{224, 2, 2};
+  if (dim == 2 && law == LAW_SW) return FdCfg{160, nq <= 5 ? 4 : 3, 1};
+  // (Nq = 4, FP64: 136 registers without a bound, two CTAs all the same; held to 128 it
+  // spills, 8x8 elements at 10 LSRK54 steps 173 -> 179 us)
+  if (dim == 2) return FdCfg{224, nq == 4 && vk == VK_EC ? 1 : 2, 2};
   // weak form: little arithmetic, so more CTAs for the memory (24^3 elements, N =
   // 4: 75 us at 4 of 160 threads and one array, 82 at 3 and three arrays, 95 at
   // 8 of 96, 102 at 5 of 160; N = 1: 109 us at 8 of 96, 132 at 4 of 160)
@@ -106,7 +109,9 @@ __host__ __device__ constexpr FdCfg fd_cfg(int law, int dim, int vk, int nq) {
   if (nq == 7) return FdCfg{160, 3, 1};
   if (nq == 6) return FdCfg{128, 4, 1};
   if (nq == 5 || f32) return FdCfg{160, 3, f32 ? 1 : 3};
-  return FdCfg{224, 2, 3};
+  // (Nq = 4, FP64 EC: 147 registers and no spill; held to 128, ARK23 steps of 13x16x4
+  // elements take 36.7 us instead of 35.1)
+  return FdCfg{224, nq == 4 && vk == VK_EC ? 1 : 2, 3};
 }
 __host__ __device__ constexpr int line_count(int nq, int dim) { return dim * ipow(nq, dim - 1); }
 inline int fd_max_elements(int law, int dim, int vk, int nq) {
@@ -120,10 +125,12 @@ inline int fd_max_elements(int law, int dim, int vk, int nq) {
 // a full warp and the other lanes share the staging (2-D Euler-gravity N = 7,
 // 24x24 elements: 10.2 us per LSRK54 stage at 4 elements, 9.0 at 1; 3-D N = 3,
 // 6^3: 4.1 at 2, 3.6 at 1); not below 16 lines an element, where it measured
-// within 4 % either way, nor on curved elements (162 at N = 4: 8.4 us at 2, 8.9 at 1).
-inline int fd_default_elements(int nq, int dim, int emax, int K, int nsm, bool curved) {
+// within 4 % either way, on curved elements (162 at N = 4: 8.4 us at 2, 8.9 at 1), or
+// where the FP32 surface flux is chosen at run time (a copy per direction, which
+// warps of one direction run alone: 6^3 at N = 3, 6.4 us at 2, 8.0 at 1).
+inline int fd_default_elements(int nq, int dim, int emax, int K, int nsm, bool one) {
   const int nl = line_count(nq, dim);
-  if (!curved && nq >= 4 && nl >= 16 && (long long)K * ((nl + 31) / 32) <= 4LL * nsm) return 1;
+  if (one && nq >= 4 && nl >= 16 && (long long)K * ((nl + 31) / 32) <= 4LL * nsm) return 1;
   int best = emax;
   double fill = 0.0;
   for (int E = 1; E <= emax; ++E) {
@@ -203,7 +210,7 @@ inline int fd_small(int law, int dim, int vk, int nq, int sf, int K, int nsm) {
   else if (vk == VK_WEAK)
     most = nq == 4 ? 8 : nq == 5 || nq == 6 ? 3 : nq == 7 ? 2 : 0;
   else
-    most = nq == 5 ? 3 : nq >= 4 && nq <= 7 ? 2 : 0;
+    most = nq >= 4 && nq <= 7 ? 2 : 0;
   if (2LL * K > (long long)most * nsm) return 0;
   const int cap = K <= nsm ? small_threads(nq, dim) : K <= 4 * nsm ? 96 : 64;
   const int least = small_least(nq, dim), full = small_threads(nq, dim);
@@ -335,7 +342,7 @@ __device__ __forceinline__ void ec_line32(float igm1, int d, const LinePt<LAW, D
 //   longer polynomial; the core of a vortex on a coarse grid), or further apart
 //   (2: logarithms).  The form depends on the line alone, so results do not
 //   depend on the launch shape.  FP32-flux form: 0 (ec_line32), or a branch per
-//   pair (2).
+//   pair (2), which gives near pairs the same values.
 template <int LAW, int DIM, int VK, int TIER>
 __device__ __forceinline__ void line_pair(const LawP& L, double c0, int d, const LinePt<LAW, DIM, VK>& P,
                                           const LinePt<LAW, DIM, VK>& Q, double* f, double& x) {
@@ -1060,6 +1067,10 @@ __global__ void __launch_bounds__(SMALL ? small_threads(NQ, DIM) : fd_cfg(LAW, D
     }
     int form = 0;
     if constexpr (!SMALL) form = line_form<LAW, DIM, VK, NQ>(sq, sx, base, sd);
+    // FP32 flux: a warp with a line of form 2 takes it for all of them, not one form
+    // after the other (3-D N = 6, 8x6x4 elements: 115 -> 109 us per ARK23 step); a near
+    // line's pairs come out the same to the bit (tests/test_fp32flux_lines.py)
+    if constexpr (!SMALL && VK == VK_EC32 && !S::SW) form = __any_sync(0xffffffffu, form) ? 2 : 0;
     double Ts[NS];  // SMALL: the node's sums
     if constexpr (SMALL) {
       const int n0 = tid < NP ? tid : 0, i0 = n0 % NQ, i1 = n0 / NQ % NQ, i2 = n0 / (NQ * NQ);
